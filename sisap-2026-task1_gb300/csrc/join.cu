@@ -21,14 +21,30 @@
 // insertion in visit order (h desc, j asc) is then resolved by rank counting.
 //
 // Duplicates: about half of the K*K two-hop candidates of a row repeat an id
-// (1317 distinct of 2500 at 6.35M rows), so each row first inserts them into a
-// shared-memory hash table (open addressing, keys = ids).  Every occurrence of
-// an id has the same h, so h and the dot are computed once per distinct id.
-// Among the occurrences of one id only the first in visit order can change
-// the list (a later one finds the id in the list, or scores <= the threshold
-// that evicted or rejected it), and when one occurrence is selected so is the
-// first (ties at the cut are taken in j order), so the visit key of a
-// distinct id is (h, first j).
+// (1317 distinct of 2500 at 6.35M rows).  Every occurrence of an id has the
+// same h, so h and the dot are computed once per distinct id, at its first
+// occurrence (its "representative").  Among the occurrences of one id only
+// the first in visit order can change the list (a later one finds the id in
+// the list, or scores <= the threshold that evicted or rejected it), and when
+// one occurrence is selected so is the first (ties at the cut are taken in j
+// order), so the visit key of a distinct id is (h, first j).
+//
+// Finding the representatives is what the kernel used to spend most of its
+// instructions on: an open-addressing insert per occurrence (a probe loop with
+// a compare-and-swap, then an atomic for the first j) took 20k of the 38.6k
+// warp instructions of a cached row, with issue slots 61 % busy.  Now it takes
+// rounds without probing: every unresolved occurrence does one
+// atomicMin(table[hash_round(id)], tag | j); after a barrier the slot holds
+// the smallest j that hashed there, so an occurrence whose id equals the
+// winner's id has found its representative, the first occurrence, and the
+// others go to the next round with another hash.  Each round resolves at least
+// the winner of every slot, so it ends; with about 1300 ids in 4096 slots 84 %
+// resolve in the first round and three rounds are usual.  Rounds alternate
+// between two tables, so one barrier per round separates the inserts from the
+// reads, and the tag falls with every round and row, so an older entry loses
+// to any newer one and the tables are cleared once per million tags.  The
+// row's cached ids and starting list only look ids up in the same rounds: a
+// slot without this round's tag says that the id is absent.
 //
 // Across iterations a row's candidate set barely changes (over 80 % of the
 // distinct ids recur from the third iteration on), and its pool threshold
@@ -39,31 +55,33 @@
 // sketch or 2 for the optional 128-hyperplane sketch (hyperplane.cu); the
 // score is 1024 - popcount over the W words either way.
 //
-// Stages per row (shared memory, K = 50, R = 400, d = 1024: ~54 KB):
-//   A  own list, sketch, code row; clear table and histogram; start copying
-//      the row's cache entries into shared memory (cp.async); insert the
-//      starting list's ids with a real score, flagged (bit 31 of the key)
-//   B  two-hop occurrences j = k*K + k2 spread over the block (thread t takes
-//      j = t + 256r), insert each, record its slot per j and the first j per
-//      slot (atomicMin); the first occurrence to touch a slot appends it to
-//      the distinct list
-//   B2 cached h / rejected flags of the distinct ids; the rest form the miss
-//      list
-//   C  Hamming of the misses, CB in flight per 8-lane group (the autotuned
-//      candidate block): one 16-byte sketch chunk per lane (128-byte rows =
-//      one line per candidate), group __popc
-//   D  histogram of h over all occurrences, threshold h_t (warp scan)
+// Stages per row (shared memory, K = 50, R = 400, d = 1024: ~53 KB); thread t
+// owns the occurrences j = t + 256r in every stage:
+//   A  own list (loaded while the previous row was computed); the unchanged-
+//      row test; start copying the row's cache entries, code row and sketch
+//      into shared memory (cp.async)
+//   B  two-hop ids, all loaded first, then one table insert each; rounds as
+//      above: rep[j], the first-occurrence bits (registers), info[rep] of the
+//      ids found in the cache
+//   C  Hamming of the first occurrences without a cached score, each warp its
+//      own (CB in flight per 8-lane group, the autotuned candidate block): one
+//      16-byte sketch chunk per lane (128-byte rows = one line per
+//      candidate), group popcount
+//   D  histogram of h over all occurrences; every warp finds the threshold
+//      h_t from it
 //   E  selection: every occurrence with h > h_t plus the first
-//      R - count(h > h_t) occurrences with h == h_t in j order; one block scan
-//      of per-thread tie counts finds the cut position, then each distinct id
-//      is selected from its h and first j
-//   F  selected ids neither flagged as starting-list members nor known to be
-//      rejected: dp4a dots, 8 lanes per candidate; keep those above the
-//      starting pool[K-1].score, flag the others as rejected
-//   F3 write the row's cache: this iteration's distinct ids, h and flags
-//   G/H insertion by rank counting over 16-byte survivor records {visit key,
-//      dot, id, flags} (or the reference's sequential loop for an unsorted or
-//      unscored pool), write-back, update count
+//      R - count(h > h_t) occurrences with h == h_t in j order, ranked by
+//      ballot counts per (round, warp); the selected first occurrences that
+//      are neither starting-list members nor known to be rejected need a dot
+//   F  dp4a dots, 8 lanes per candidate; keep those above the starting
+//      pool[K-1].score, flag the others as rejected
+//   G  write the row's cache (this iteration's distinct ids, h and flags);
+//      insertion by rank counting over 64-bit survivor keys {dot, visit key}
+//      (or the reference's sequential loop for an unsorted or unscored pool),
+//      written straight to the output list; the update count
+// The row's bookkeeping (update count, flags, statistics) is finished by
+// thread 0 after the next row's first barrier, and what the last stage reads
+// is not written before that barrier, so a row ends without one.
 // Per row HBM/L2 bytes: K*8 (own list) + K*K*4 (two-hop ids) + d + d/8 (own
 // row, sketch) + U*d/8 (U sketches scored) + r*d (r reranked rows) + 12 per
 // distinct id (cache read and write).
@@ -81,52 +99,157 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kGroups = kThreads / 8;  // 8-lane groups per CTA
-constexpr int kHBins = 1025;
-static_assert(kHBins * 4 >= kCacheCap * 2, "the histogram region stages the cached scores");
-constexpr int32_t kEmpty = 0x7fffffff;     // never a valid id (num_trees * n < 2^31)
-constexpr uint32_t kPoolFlag = 0x80000000u; // key bit: id is in the starting list with a real score
-constexpr uint32_t kFirstMask = 0x1fffu;    // meta bits 0..12: first j (8191 = none); 16..26: Hamming score
-constexpr uint32_t kKnown = 0x80000000u;    // meta bit 31: Hamming score taken from the row's candidate cache
-constexpr uint32_t kRej = 0x40000000u;      // meta bit 30: dot known to be <= the row's pool threshold
+constexpr int kHBins = 1152;           // distances 0..1024, padded to 9 x 128 for the threshold scan
+constexpr uint32_t kNoDist = kHBins - 1;     // "distance" of an occurrence without a candidate: behind every real one
+constexpr int kMaxPairs = (kMaxK * kMaxK / 2 + kThreads - 1) / kThreads;  // occurrence pairs per thread
+constexpr int kCachePairs = kCacheCap / 2 / kThreads;                     // pairs of cached ids per thread
+static_assert(kCacheCap % (2 * kThreads) == 0, "cached ids per thread");
+constexpr uint32_t kJBits = 12;              // occurrence index j < kMaxK * kMaxK
+constexpr uint32_t kJMask = (1u << kJBits) - 1u;
+static_assert(kMaxK * kMaxK <= (1 << kJBits), "occurrence index");
+constexpr uint32_t kTagTop = 0xffffeu;       // tags count down from here; 0xfffff marks a cleared slot
+constexpr int kTableB = 1024;                // second table (odd rounds): slots
+constexpr int kTableBShift = 22;
+constexpr uint32_t kXMask = 0x7ffu;          // info bits 0..10: Hamming distance
+constexpr uint32_t kKnown = 0x800u;          // info bit 11: distance taken from the row's candidate cache
+constexpr uint32_t kRej = 0x1000u;           // info bit 12: dot known to be <= the row's pool threshold
+constexpr uint32_t kNone = 0xffffffffu;      // ids: no candidate (no id equals it: num_trees * n < 2^31)
+constexpr uint32_t kPoolFlag = 0x80000000u;  // ids bit 31: the id is in the starting list with a real score
+// The default parameters get a kernel of their own whose sizes and
+// shared-memory offsets are compile-time constants: read from the parameter
+// block they cost about 4,000 more instructions per row.
+constexpr int kDefK = 50, kDefR = 400;
 
-struct JoinSmem {
-  int K, R, KK, d, W, HT;
-  size_t bytes;
-  size_t o_code, o_sk, o_slot, o_key, o_meta, o_hist, o_ulist, o_surv, o_pool_id, o_pool_sc, o_miss;
+// Shared-memory layout of one CTA (byte offsets).
+struct JoinLayout {
+  int KK;                  // K * K occurrences
+  int pairs;               // pairs of consecutive occurrences
+  int ta_slots, ta_shift;  // first table: slots and hash shift
+  uint32_t kdiv;           // j / K = (j * kdiv) >> 20 for j < 4096
+  uint32_t dummy;          // info index of occurrences without a candidate
+  uint32_t o_code, o_sk, o_ids, o_rep, o_info, o_ta, o_tb, o_hist, o_x, o_pool, o_row, o_cell;
+  uint32_t bytes;
 };
 
-__host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
+__host__ __device__ constexpr uint32_t align16(uint32_t x) { return (x + 15u) & ~15u; }
+__host__ __device__ constexpr uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
-__host__ __device__ inline JoinSmem join_smem(int K, int R, int d) {
-  JoinSmem s;
-  s.K = K;
-  s.R = R;
+__host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d) {
+  JoinLayout s{};
   s.KK = K * K;
-  s.d = d;
-  s.W = d / 64;  // room for the widest sketch (the sign sketch); a hyperplane sketch uses 2 words
-  s.HT = 1024;
-  while (s.HT < (3 * (s.KK + K)) / 2) s.HT <<= 1;  // load factor <= 2/3
-  size_t o = 0;
-  s.o_code = o;    o = align16(o + size_t(d));
-  s.o_sk = o;      o = align16(o + size_t(s.W) * 8);
-  s.o_slot = o;    o = align16(o + size_t(s.KK) * 2);
-  s.o_key = o;     o = align16(o + size_t(s.HT) * 4);
-  s.o_meta = o;    o = align16(o + size_t(s.HT) * 4);
-  s.o_hist = o;    o = align16(o + size_t(kHBins) * 4);
-  s.o_ulist = o;   o = align16(o + size_t(s.KK) * 2);
-  const size_t u0 = o;  // stage C's miss list shares this region with stages F-H
-  s.o_surv = o;    o = align16(o + size_t(R) * 16);  // survivors {visit key, dot, id, flags}
-  s.o_miss = u0;  // also stages the row's cached ids (kCacheCap * 4 bytes) before stage B2
-  if (o < align16(u0 + size_t(s.KK) * 2)) o = align16(u0 + size_t(s.KK) * 2);
-  if (o < align16(u0 + size_t(kCacheCap) * 4)) o = align16(u0 + size_t(kCacheCap) * 4);
-  s.o_pool_id = o; o = align16(o + size_t(K) * 4);
-  s.o_pool_sc = o; o = align16(o + size_t(K) * 4);
+  s.pairs = (s.KK + 1) / 2;
+  s.kdiv = ((1u << 20) + uint32_t(K) - 1) / uint32_t(K);
+  // first table: 4096 slots for K = 50 (at most 2500 ids, about 1300 usual)
+  s.ta_slots = 1024;
+  s.ta_shift = 22;
+  while (s.ta_slots < (3 * (s.KK + K)) / 2) {
+    s.ta_slots <<= 1;
+    --s.ta_shift;
+  }
+  const uint32_t kk = uint32_t(2 * s.pairs), r = uint32_t(R);
+  s.dummy = align16(2 * kk) / 2;
+  uint32_t o = 0;
+  s.o_ids = o;   o += align16(4 * kk);
+  s.o_rep = o;   o += align16(umax(2 * kk, 14 * r));  // representatives, then the survivors' keys, ids and order
+  s.o_info = o;  o += align16(2 * kk) + 16;
+  s.o_ta = o;    o += uint32_t(s.ta_slots) * 4;
+  s.o_tb = o;    o += kTableB * 4;
+  s.o_hist = o;  o += kHBins * 4;  // also the row's cached distances, staged and gathered
+  // staged cached ids, then the warps' miss lists, then the rerank list, then
+  // the ids of the row's next cache
+  s.o_x = o;     o += align16(umax(umax(kCacheCap * 4, uint32_t((s.pairs + kThreads - 1) / kThreads) * kThreads * 4), 2 * r));
+  s.o_pool = o;  o += 2 * 2 * kMaxK * 4;  // starting lists of this row and of the previous one: ids, scores
+  s.o_row = o;   o += 2 * 32;             // row counters, by row parity
+  s.o_cell = o;  o += kMaxPairs * kWarps * 4;  // threshold ties per (round, warp)
+  s.o_sk = o;    o += 128;                // the widest sketch
+  s.o_code = o;  o += align16(uint32_t(d));
   s.bytes = o;
   return s;
 }
+static_assert(kHBins * 4 >= kCacheCap * 2, "the histogram region stages the cached distances");
 
-__device__ __forceinline__ int popc_u4(uint4 a, uint4 b) {
-  return __popc(a.x ^ b.x) + __popc(a.y ^ b.y) + __popc(a.z ^ b.z) + __popc(a.w ^ b.w);
+// A row's counters (byte offsets from its set's start).
+enum : uint32_t {
+  kRowCnt = 0,       // occurrences with a candidate
+  kRowNu = 4,        // distinct candidates
+  kRowMiss = 8,      // of these without a cached distance
+  kRowNeed = 12,     // selected ones that need a dot
+  kRowProm = 16,     // survivors
+  kRowChanged = 20,  // list positions whose id changed
+};
+
+// Shared memory is addressed through one 32-bit base register: with C++
+// pointers into the dynamic array the compiler recomputed the window's base
+// (three to four uniform instructions) at most of the accesses, about 5,000
+// instructions per row.
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void sts16(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"(uint16_t(v)) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void red_min(uint32_t a, uint32_t v) {
+  asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_min_if(bool p, uint32_t a, uint32_t v) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q red.shared.min.u32 [%0], %1;\n}" ::"r"(a), "r"(v), "r"(uint32_t(p))
+               : "memory");
+}
+__device__ __forceinline__ void sts16_if(bool p, uint32_t a, uint32_t v) {
+  asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q st.shared.u16 [%0], %1;\n}" ::"r"(a), "h"(uint16_t(v)), "r"(uint32_t(p))
+               : "memory");
+}
+__device__ __forceinline__ void red_add(uint32_t a, uint32_t v) {
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t atom_add(uint32_t a, uint32_t v) {
+  uint32_t o;
+  asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
+  return o;
+}
+// 16-byte global -> shared copy that holds no registers (cp.async, L2 only).
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// Popcount of four words with three popc instructions: a carry-save adder
+// turns three of them into a sum and a carry word (popc runs at a quarter of
+// the rate of logic instructions).
+__device__ __forceinline__ uint32_t popc_u4(uint4 a, uint4 b) {
+  const uint32_t x = a.x ^ b.x, y = a.y ^ b.y, z = a.z ^ b.z, w = a.w ^ b.w;
+  const uint32_t sum = x ^ y ^ z, carry = (x & y) | (x & z) | (y & z);
+  return uint32_t(__popc(sum) + __popc(w) + 2 * __popc(carry));
 }
 
 __device__ __forceinline__ int dot_u4(uint4 a, uint4 b, int acc) {
@@ -136,601 +259,792 @@ __device__ __forceinline__ int dot_u4(uint4 a, uint4 b, int acc) {
   return __dp4a(int(a.w), int(b.w), acc);
 }
 
-__device__ __forceinline__ uint32_t hash_slot(int32_t id, uint32_t mask) {
-  return (uint32_t(id) * 2654435761u >> 7) & mask;
+// A lane's share of the dot of a code row (its 16-byte chunks 128 bytes apart
+// from `row` on) with the row in shared memory.
+template <int CHUNKS>
+__device__ __forceinline__ int dot_lane(const int8_t* row, uint32_t mine) {
+  uint4 x[CHUNKS];
+  int acc = 0;
+#pragma unroll
+  for (int u = 0; u < CHUNKS; ++u) x[u] = __ldg(reinterpret_cast<const uint4*>(row + 128 * u));
+#pragma unroll
+  for (int u = 0; u < CHUNKS; ++u) acc = dot_u4(x[u], lds128(mine + 128 * u), acc);
+  return acc;
 }
 
-// Find or insert id (flagged keys match by their low 31 bits).  The table
-// always has free slots (load <= 2/3), so the probe ends; the bound is a guard.
-__device__ __forceinline__ int table_insert(int32_t* key, uint32_t mask, int32_t id, uint32_t flag) {
-  uint32_t s = hash_slot(id, mask);
-  for (uint32_t probe = 0; probe <= mask; ++probe) {
-    int32_t k = key[s];
-    if (k == kEmpty) {
-      const int32_t prev = atomicCAS(&key[s], kEmpty, int32_t(uint32_t(id) | flag));
-      if (prev == kEmpty) return int(s);
-      k = prev;
-    }
-    if ((uint32_t(k) & 0x7fffffffu) == uint32_t(id)) return int(s);
-    s = (s + 1) & mask;
+// Byte offset of id's slot in a table of 2^(32 - shift) words, round 0 or
+// later: a multiplicative hash whose odd multiplier changes with the round,
+// so ids that met in one round part in the next.
+__device__ __forceinline__ uint32_t slot_of(uint32_t id, uint32_t round, int shift) {
+  return ((id * (2654435761u + round * 0x3C6EF372u)) >> shift) << 2;
+}
+
+__device__ __forceinline__ int warp_incl_scan(int v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
   }
-  return -1;
+  return v;
 }
 
-// 16-byte global -> shared copy that holds no registers (cp.async, L2 only).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// Slot of id (flagged or not), or -1 when the table does not hold it.
-__device__ __forceinline__ int table_find(const int32_t* key, uint32_t mask, int32_t id) {
-  uint32_t s = hash_slot(id, mask);
-  for (uint32_t probe = 0; probe <= mask; ++probe) {
-    const int32_t k = key[s];
-    if (k == kEmpty) return -1;
-    if ((uint32_t(k) & 0x7fffffffu) == uint32_t(id)) return int(s);
-    s = (s + 1) & mask;
-  }
-  return -1;
-}
-
-template <int CB, int MINB>
+// CB: sketches in flight per 8-lane group (Hamming stage); MINB: resident CTAs
+// per SM the register budget allows; DEF: the default K and R (and 8-byte
+// aligned input lists), else any.
+template <int CB, int MINB, bool DEF>
 __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
-    const int8_t* __restrict__ codes, const uint64_t* __restrict__ sketch, int64_t n, int d, int K, int R, int W,
+    const int8_t* __restrict__ codes, const uint64_t* __restrict__ sketch, int64_t n64, int d, int K_, int R_, int W,
     const int32_t* ids_in, const int32_t* scores_in, int32_t* ids_out, int32_t* scores_out,
-    const int32_t* __restrict__ row_order, unsigned long long* __restrict__ counters, JobTable jt, JoinCtl ctl) {
+    const int32_t* __restrict__ row_order, unsigned long long* __restrict__ counters, JobTable jt, JoinCtl ctl,
+    const JoinLayout LA) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (ctl.all_done && *reinterpret_cast<volatile int*>(ctl.all_done)) return;
-  const JoinSmem L = join_smem(K, R, d);
-  uint4* my_code = reinterpret_cast<uint4*>(smem + L.o_code);
-  uint4* my_sk = reinterpret_cast<uint4*>(smem + L.o_sk);
-  int16_t* cand_slot = reinterpret_cast<int16_t*>(smem + L.o_slot);
-  int32_t* key = reinterpret_cast<int32_t*>(smem + L.o_key);
-  uint32_t* meta = reinterpret_cast<uint32_t*>(smem + L.o_meta);
-  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + L.o_hist);
-  int16_t* ulist = reinterpret_cast<int16_t*>(smem + L.o_ulist);
-  int16_t* need = cand_slot;  // stage F: the occurrence slots are dead after stage E
-  int16_t* misslist = reinterpret_cast<int16_t*>(smem + L.o_miss);  // shares its region with need..order
-  const int32_t* stage_id = reinterpret_cast<const int32_t*>(smem + L.o_miss);  // stage A..B2, same region
-  const uint16_t* stage_hr = reinterpret_cast<const uint16_t*>(smem + L.o_hist);  // stage A..B2
-  int4* surv = reinterpret_cast<int4*>(smem + L.o_surv);
-  uint16_t* order = reinterpret_cast<uint16_t*>(cand_slot);  // serial insertion, after stage F
-  int32_t* pool_id = reinterpret_cast<int32_t*>(smem + L.o_pool_id);
-  int32_t* pool_sc = reinterpret_cast<int32_t*>(smem + L.o_pool_sc);
-  __shared__ int s_cnt, s_ht, s_gt, s_jcut, s_nu, s_nneed, s_nprom, s_nmiss, s_ccnt;
-  __shared__ int32_t s_wsum[kWarps], s_wsum2[kWarps];
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7, slot8 = lane >> 3;
-  const int KK = L.KK, nchunk = d / 16, sk_chunks = W / 2;  // W: sketch words per row (<= L.W = d / 64)
-  const uint32_t mask = uint32_t(L.HT - 1);
+  constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim);
+#define KNNG_L(f) (DEF ? LD.f : LA.f)
+  constexpr int NP = DEF ? (LD.pairs + kThreads - 1) / kThreads : kMaxPairs;  // pairs per thread
+  const int K = DEF ? kDefK : K_, R = DEF ? kDefR : R_;
+  uint32_t sb, tid_;
+  asm volatile("{\n.reg .u64 t;\ncvta.to.shared.u64 t, %1;\ncvt.u32.u64 %0, t;\n}" : "=r"(sb) : "l"(smem));
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid_));
+  const int tid = int(tid_);
+  const unsigned full = 0xffffffffu;
+  const int lane = tid & 31, warp = tid >> 5, sub = lane & 7, slot8 = lane >> 3;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint32_t n = uint32_t(n64);  // num_trees * n fits in int32
+  const int sk_chunks = W / 2;       // W: sketch words per row
   const bool inplace = ids_out == ids_in;
   const bool cached = ctl.cache_ids != nullptr;
+  const uint32_t a_ids = sb + KNNG_L(o_ids), a_rep = sb + KNNG_L(o_rep), a_info = sb + KNNG_L(o_info);
+  const uint32_t a_ta = sb + KNNG_L(o_ta), a_tb = sb + KNNG_L(o_tb), a_hist = sb + KNNG_L(o_hist);
+  const uint32_t a_x = sb + KNNG_L(o_x), a_cell = sb + KNNG_L(o_cell), a_code = sb + KNNG_L(o_code);
+  // survivors: 64-bit keys {dot, visit key}, then ids, then (sequential insertion) their visit order
+  const uint32_t a_sid = a_rep + 8u * uint32_t(R), a_sorder = a_rep + 12u * uint32_t(R);
   // per-CTA statistics, kept by thread 0 in shared memory (no registers held
   // across the row loop): updates, sketches scored, rows reranked, distinct
   // candidates, rows skipped
   __shared__ unsigned long long s_stat[5];
-  if (tid == 0)
+  __shared__ unsigned long long s_run_upd;  // updates of job s_run_job not yet added to its count
+  __shared__ int s_run_job;
+  __shared__ int s_pend_i, s_pend_job;      // the computed row whose bookkeeping is still open, and its job
+  __shared__ int s_job[2];                  // job of the row in each list buffer (thread 0)
+  if (tid == 0) {
     for (int q = 0; q < 5; ++q) s_stat[q] = 0;
-  int run_job = -1;                 // per-job update count kept by warp 0 lane 0
-  unsigned long long run_upd = 0;
+    s_run_upd = 0;
+    s_run_job = -1;
+    s_pend_i = -1;
+    s_job[0] = s_job[1] = 0;
+  }
+  if (tid < 16) sts32(sb + KNNG_L(o_row) + 4 * tid, 0);
+  if (tid == 0) sts16(a_info + 2 * KNNG_L(dummy), kNoDist);
+  auto clear_tables = [&]() {
+    const uint4 e = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int t = tid; t < KNNG_L(ta_slots) / 4; t += kThreads) sts128(a_ta + 16 * t, e);
+    for (int t = tid; t < kTableB / 4; t += kThreads) sts128(a_tb + 16 * t, e);
+  };
+  clear_tables();
+  uint32_t tag = kTagTop;           // block-uniform
+  uint32_t par = 0;                 // parity of the computed rows
 
-  // job_done only changes between launches, so a CTA reads each job's flag
-  // once; the next row's index is fetched one row ahead
-  int flag_job = -1, flag_done = 0;
-  const int64_t nrows = (ctl.row_limit > 0 && ctl.row_limit < n) ? ctl.row_limit : n;
-  int64_t next_i = int64_t(blockIdx.x) < nrows ? (row_order ? int64_t(row_order[blockIdx.x]) : int64_t(blockIdx.x)) : 0;
-  for (int64_t r = blockIdx.x; r < nrows; r += gridDim.x) {
-    const int64_t i = next_i;
-    if (r + gridDim.x < nrows) next_i = row_order ? int64_t(row_order[r + gridDim.x]) : r + gridDim.x;
-    if (!KNNG_GUARD(ctl.check_err, i >= 0 && i < n)) continue;  // block-uniform
-    int job = 0;
-    if (ctl.job_done) {
-      job = job_of(jt, i);
-      if (job != flag_job) {
-        flag_job = job;
-        flag_done = ctl.job_done[job];
+  // Bookkeeping of the last computed row, by thread 0 once a barrier has
+  // passed since its last stage; frees its counters for the row after next.
+  auto finish_row = [&]() {
+    if (tid != 0 || s_pend_i < 0) return;
+    const uint32_t c = sb + KNNG_L(o_row) + 32u * (par ^ 1u);
+    const uint4 u = lds128(c);
+    const uint2 w = lds64(c + kRowProm);
+    sts128(c, make_uint4(0, 0, 0, 0));
+    sts64(c + kRowProm, 0, 0);
+    s_stat[0] += w.y;
+    s_stat[1] += u.z;
+    s_stat[2] += u.w;
+    s_stat[3] += u.y;
+    if (ctl.chg_out) ctl.chg_out[s_pend_i] = w.y ? 1 : 0;
+    if (ctl.job_upd) {
+      if (s_pend_job != s_run_job) {
+        if (s_run_job >= 0 && s_run_upd) atomicAdd(ctl.job_upd + s_run_job, s_run_upd);
+        s_run_job = s_pend_job;
+        s_run_upd = 0;
       }
-      if (flag_done) {  // stopped job: its rows pass through unchanged
-        if (!inplace)
-          for (int k = tid; k < K; k += kThreads) {
-            ids_out[i * K + k] = ids_in[i * K + k];
-            scores_out[i * K + k] = scores_in[i * K + k];
-          }
-        continue;
+      s_run_upd += w.y;
+    }
+    s_pend_i = -1;
+  };
+
+  // A row's index is loaded two rows ahead; its own list (cp.async into the
+  // other list buffer), cache count, change flags and its job's state while
+  // the row before is computed.  The flags are combined at the row's start, so
+  // nothing waits for them before.
+  const int nrows = int((ctl.row_limit > 0 && ctl.row_limit < n64) ? ctl.row_limit : n64);
+  auto row_at = [&](int r) { return r < nrows && r >= 0 ? (row_order ? row_order[r] : r) : -1; };
+  int32_t nx_i = row_at(blockIdx.x), nx2_i = row_at(int(blockIdx.x) + int(gridDim.x));
+  uint32_t slot = 0;                    // list buffer of the current row
+  int nx_cc = 0, nx_flag = 0, nx_done = 0;
+  auto fetch_list = [&](uint32_t to) {  // list and cache count of row nx_i
+    if (nx_i >= 0 && KNNG_GUARD(ctl.check_err, nx_i < int(n))) {
+      if (tid < K) {
+        const uint32_t dst = sb + KNNG_L(o_pool) + to * (2u * kMaxK * 4u) + 4u * uint32_t(tid);
+        cp_async4(dst, ids_in + int64_t(nx_i) * K + tid);
+        cp_async4(dst + kMaxK * 4u, scores_in + int64_t(nx_i) * K + tid);
       }
+      if (cached) nx_cc = ctl.cache_cnt[nx_i];
+    }
+    cp_async_commit();
+  };
+  // (unchanged-row skip, double-buffered iterations only) a row whose own
+  // list and every neighbour's list came out of the previous iteration
+  // unchanged sees exactly the inputs it saw then, so its result is its
+  // current list: it is copied through without any work, as are the rows of a
+  // stopped job
+  auto fetch_flags = [&](uint32_t to) {
+    cp_async_wait_all();
+    nx_flag = nx_done = 0;
+    if (tid <= K && nx_i >= 0 && (!kChecked || nx_i < int(n))) {
+      nx_flag = 1;
+      if (ctl.chg_in) {
+        const uint32_t at = tid < K ? lds32(sb + KNNG_L(o_pool) + to * (2u * kMaxK * 4u) + 4u * uint32_t(tid)) : uint32_t(nx_i);
+        if (at < n) nx_flag = int(ctl.chg_in[at]);
+      }
+      if (ctl.job_done) {
+        const int job = job_of(jt, nx_i);
+        nx_done = ctl.job_done[job];
+        if (tid == 0) s_job[to] = job;
+      }
+    }
+  };
+  fetch_list(0);
+  fetch_flags(0);
+  for (int r0 = int(blockIdx.x); r0 < nrows && r0 >= 0; r0 += int(gridDim.x), slot ^= 1u) {
+    const int i = nx_i;
+    const int cc = cached ? min(nx_cc, ctl.cache_cap) : 0;
+    const int moved = nx_done ? 0 : nx_flag;
+    const int stopped = nx_done;  // threads 0..K
+    nx_i = nx2_i;
+    nx2_i = row_at(r0 + 2 * int(gridDim.x));
+    if (i < 0 || !KNNG_GUARD(ctl.check_err, i < int(n))) {  // block-uniform
+      KNNG_FLAG_IF(ctl.check_err, i < 0);
+      __syncthreads();  // the other list buffer may still be read
+      fetch_list(slot ^ 1u);
+      fetch_flags(slot ^ 1u);
+      continue;
     }
     // ---- A
-    // (unchanged-row skip, double-buffered iterations only) a row whose own
-    // list and every neighbour's list came out of the previous iteration
-    // unchanged sees exactly the inputs it saw then, so its result is its
-    // current list: it is copied through without any work
-    int moved = ctl.chg_in ? 0 : 1;
-    for (int k = tid; k < K; k += kThreads) {
-      const int32_t id = ids_in[i * K + k];
-      pool_id[k] = id;
-      pool_sc[k] = scores_in[i * K + k];
-      KNNG_FLAG_IF(ctl.check_err, id < 0 || id >= n);
-      if (ctl.chg_in) moved |= (id < 0 || id >= n) ? 1 : int(ctl.chg_in[id]);
-    }
-    if (ctl.chg_in && tid == 0) moved |= int(ctl.chg_in[i]);
-    if (!cached)
-      for (int h = tid; h < kHBins; h += kThreads) hist[h] = 0;
-    for (int t = tid; t < L.HT / 4; t += kThreads) {
-      reinterpret_cast<uint4*>(key)[t] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
-      reinterpret_cast<uint4*>(meta)[t] = make_uint4(kFirstMask, kFirstMask, kFirstMask, kFirstMask);
-    }
-    if (tid == 0) {
-      s_cnt = 0;
-      s_nu = 0;
-      s_nneed = 0;
-      s_nprom = 0;
-      s_ccnt = cached ? ctl.cache_cnt[i] : 0;
-    }
-    if (__syncthreads_or(moved) == 0) {  // block-uniform
-      for (int k = tid; k < K; k += kThreads) {  // from global memory: the shared copies may be reused at once
-        ids_out[i * K + k] = ids_in[i * K + k];
-        scores_out[i * K + k] = scores_in[i * K + k];
+    const uint32_t a_pool = sb + KNNG_L(o_pool) + slot * (2u * kMaxK * 4u);  // ids; scores kMaxK words on
+    const uint32_t a_psc = a_pool + kMaxK * 4u;
+    const uint32_t a_row = sb + KNNG_L(o_row) + 32u * par;
+    const bool work = __syncthreads_or(moved) != 0;  // block-uniform
+    finish_row();
+    if (!work) {
+      if (!inplace && tid < K) {
+        ids_out[int64_t(i) * K + tid] = int32_t(lds32(a_pool + 4 * tid));
+        scores_out[int64_t(i) * K + tid] = int32_t(lds32(a_psc + 4 * tid));
       }
-      if (tid == 0) {
+      if (tid == 0 && !stopped) {
         ctl.chg_out[i] = 0;
         ++s_stat[4];
       }
+      fetch_list(slot ^ 1u);
+      fetch_flags(slot ^ 1u);
       continue;
     }
-    for (int c = tid; c < nchunk; c += kThreads) my_code[c] = reinterpret_cast<const uint4*>(codes + i * d)[c];
-    for (int c = tid; c < sk_chunks; c += kThreads) my_sk[c] = reinterpret_cast<const uint4*>(sketch + i * W)[c];
-    if (cached) {
-      // stage the row's cache entries into shared memory (ids over the region
-      // of stages F-H, scores over the histogram) while stage B runs; the
-      // rows' cache slices are 16-byte aligned and sized for cache_cap
-      const int cc = min(s_ccnt, ctl.cache_cap);
+    // own code row and sketch, and the row's cache entries (ids over the miss
+    // list, distances over the histogram); the rows' cache slices are 16-byte
+    // aligned and sized for cache_cap
+    {
+      const int nchunk = d / 16;
       const int n_id = (cc * 4 + 15) / 16, n_hr = (cc * 2 + 15) / 16;
-      const char* gid = reinterpret_cast<const char*>(ctl.cache_ids + i * ctl.cache_cap);
-      const char* ghr = reinterpret_cast<const char*>(ctl.cache_hr + i * ctl.cache_cap);
-      for (int t = tid; t < n_id + n_hr; t += kThreads) {
-        if (t < n_id) cp_async16(smem + L.o_miss + 16 * t, gid + 16 * t);
-        else cp_async16(smem + L.o_hist + 16 * (t - n_id), ghr + 16 * (t - n_id));
-      }
+      const char* gid = reinterpret_cast<const char*>(ctl.cache_ids + int64_t(i) * ctl.cache_cap);
+      const char* ghr = reinterpret_cast<const char*>(ctl.cache_hr + int64_t(i) * ctl.cache_cap);
+      for (int t = tid; t < n_id; t += kThreads) cp_async16(a_x + 16 * t, gid + 16 * t);
+      for (int t = tid; t < n_hr; t += kThreads) cp_async16(a_hist + 16 * t, ghr + 16 * t);
+      if (tid < nchunk) cp_async16(a_code + 16 * tid, codes + int64_t(i) * d + 16 * tid);
+      else if (tid - nchunk < sk_chunks)
+        cp_async16(sb + KNNG_L(o_sk) + 16 * (tid - nchunk),
+                   reinterpret_cast<const char*>(sketch + int64_t(i) * W) + 16 * (tid - nchunk));
       cp_async_commit();
     }
-    int irregular = 0;
-    for (int k = tid; k < K; k += kThreads) {
-      const int32_t id = pool_id[k];
-      if (pool_sc[k] != kScoreMinI && id >= 0 && id < n) table_insert(key, mask, id, kPoolFlag);
-      irregular |= (pool_sc[k] == kScoreMinI) | (k + 1 < K && pool_sc[k] < pool_sc[k + 1]);
-    }
-    // An unscored entry (INT32_MIN, tiny inputs only) can share its id with a
-    // survivor, and an unsorted pool (possible through the stage entry point)
-    // breaks the rank formulas of stage G/H: both take the sequential loop.
-    const bool serial_insert = __syncthreads_or(irregular) != 0;
-    // ---- B  two-hop occurrences j = k*K + k2 spread over the block (thread t
-    //         takes j = t + 256r), all loaded first; the first occurrence to
-    //         touch a slot appends it to the distinct list
-    {
-      constexpr int kRounds = (kMaxK * kMaxK + kThreads - 1) / kThreads;
-      const uint32_t kdiv = ((1u << 20) + uint32_t(K) - 1) / uint32_t(K);  // j / K = (j * kdiv) >> 20 for j < 4096
-      int32_t v[kRounds];
-#pragma unroll
-      for (int t = 0; t < kRounds; ++t) {
-        const int j = tid + kThreads * t;
-        int32_t val = -1;
-        if (j < KK) {
-          const int k = int((uint32_t(j) * kdiv) >> 20);
-          const int32_t n1 = pool_id[k];
-          if (n1 >= 0 && n1 < n) {
-            val = ids_in[int64_t(n1) * K + (j - k * K)];
-            KNNG_FLAG_IF(ctl.check_err, val < 0 || val >= n);
-          }
-        }
-        v[t] = val;
-      }
-      int local_cnt = 0;
-#pragma unroll
-      for (int t = 0; t < kRounds; ++t) {
-        const int j = tid + kThreads * t;
-        if (kThreads * t >= KK) break;  // block-uniform: no occurrence left for any thread
-        const int32_t n2 = v[t];
-        int sl = -1;
-        bool first = false;
-        if (j < KK) {
-          if (n2 >= 0 && n2 < n && n2 != i) sl = table_insert(key, mask, n2, 0u);
-          cand_slot[j] = int16_t(sl);
-          if (sl >= 0) {
-            // rounds visit j in increasing order, so once a slot records a
-            // smaller first j (a plain read suffices) this occurrence is not
-            // the first; otherwise the atomic decides, and exactly one of the
-            // threads that saw the slot untouched gets kFirstMask back
-            if (meta[sl] > uint32_t(j)) first = atomicMin(&meta[sl], uint32_t(j)) == kFirstMask;
-            ++local_cnt;
-          }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, first);
-        int base = 0;
-        if (lane == 0 && bal) base = atomicAdd(&s_nu, __popc(bal));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (first) ulist[base + __popc(bal & ((1u << lane) - 1u))] = int16_t(sl);
-      }
-      if (local_cnt) atomicAdd(&s_cnt, local_cnt);
-    }
-    if (cached) cp_async_wait_all();  // this thread's staging copies (stage A); the barrier publishes them
-    __syncthreads();
-    const int nu = s_nu;
-    // ---- B2  candidate cache: the row's distinct candidates of the previous
-    //          iteration with their Hamming scores and rejected flags.  Entries
-    //          are only looked up (no slot is added), and a distinct id of this
-    //          iteration without an entry goes to the miss list for stage C.
-    const int16_t* clist = ulist;
-    int ncl = nu;
-    if (cached) {
-      const int cc = min(s_ccnt, ctl.cache_cap);
-      for (int q = tid; q < cc; q += kThreads) {
-        const int sl = table_find(key, mask, stage_id[q]);
-        if (sl >= 0) {
-          const uint32_t hr = stage_hr[q];
-          meta[sl] = kKnown | ((hr & 1u) ? kRej : 0u) | (uint32_t(hr >> 1) << 16) | (meta[sl] & kFirstMask);
-        }
-      }
-      if (tid == 0) s_nmiss = 0;
+    if (tag < uint32_t(KNNG_L(KK)) + 16u) {  // a row uses at most KK + 1 tags; block-uniform, once per ~300,000 rows
+      clear_tables();
+      tag = kTagTop;
       __syncthreads();
-      for (int h = tid; h < kHBins; h += kThreads) hist[h] = 0;  // the staged scores are consumed
-      for (int q0 = warp * 32; q0 < nu; q0 += kThreads) {
-        const int q = q0 + lane;
-        const int sl = q < nu ? int(ulist[q]) : -1;
-        const bool miss = sl >= 0 && !(meta[sl] & kKnown);
-        const unsigned bal = __ballot_sync(0xffffffffu, miss);
-        int base = 0;
-        if (lane == 0 && bal) base = atomicAdd(&s_nmiss, __popc(bal));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (miss) misslist[base + __popc(bal & ((1u << lane) - 1u))] = int16_t(sl);
-      }
-      __syncthreads();
-      clist = misslist;
-      ncl = s_nmiss;
     }
-    // ---- C  Hamming once per distinct id without a cached score (groups of 8
-    //         lanes, CB candidates in flight per group)
-    {
-      const uint4 mine = sub < sk_chunks ? my_sk[sub] : make_uint4(0, 0, 0, 0);
-      for (int wbase = warp * 4; wbase < ncl; wbase += CB * kGroups) {
-        const int base = wbase + slot8;
-        uint4 v[CB];
-        int sl[CB];
+    // ---- B  two-hop occurrences, pair p = tid + 256r holding j = 2p, 2p + 1;
+    //         all loaded first
+    uint32_t v[2 * NP];
 #pragma unroll
-        for (int u = 0; u < CB; ++u) {
-          const int q = base + u * kGroups;
-          sl[u] = q < ncl ? int(clist[q]) : -1;
-          v[u] = make_uint4(0, 0, 0, 0);
-          if (sl[u] >= 0 && sub < sk_chunks) {
-            const int32_t id = int32_t(uint32_t(key[sl[u]]) & 0x7fffffffu);
-            v[u] = __ldg(reinterpret_cast<const uint4*>(sketch + int64_t(id) * W) + sub);
+    for (int r = 0; r < NP; ++r) {
+      const int p = tid + kThreads * r;
+      v[2 * r] = v[2 * r + 1] = ~0u;
+      if (DEF) {  // a pair lies in one list and is 8-byte aligned
+        if (p < LD.pairs) {
+          const int k = p / (kDefK / 2);
+          const uint32_t n1 = lds32(a_pool + 4 * k);
+          if (n1 < n) {
+            const int2 g = *reinterpret_cast<const int2*>(ids_in + int64_t(n1) * kDefK + 2 * (p - k * (kDefK / 2)));
+            v[2 * r] = uint32_t(g.x);
+            v[2 * r + 1] = uint32_t(g.y);
+            KNNG_FLAG_IF(ctl.check_err, v[2 * r] >= n || v[2 * r + 1] >= n);
           }
         }
+      } else {
 #pragma unroll
-        for (int u = 0; u < CB; ++u) {
-          int pc = (sl[u] >= 0 && sub < sk_chunks) ? popc_u4(v[u], mine) : 0;
-          pc += __shfl_xor_sync(0xffffffffu, pc, 1);
-          pc += __shfl_xor_sync(0xffffffffu, pc, 2);
-          pc += __shfl_xor_sync(0xffffffffu, pc, 4);
-          if (sub == 0 && sl[u] >= 0) meta[sl[u]] = (uint32_t(1024 - pc) << 16) | (meta[sl[u]] & kFirstMask);
-        }
-      }
-    }
-    __syncthreads();
-    // ---- D  histogram over occurrences, threshold
-    for (int j = tid; j < KK; j += kThreads) {
-      const int sl = cand_slot[j];
-      if (sl >= 0) atomicAdd(&hist[(meta[sl] >> 16) & 0x7ffu], 1u);
-    }
-    __syncthreads();
-    const int cnt = s_cnt;
-    if (tid == 0) {
-      s_stat[1] += unsigned(ncl);
-      s_stat[3] += unsigned(nu);
-    }
-    if (cnt > R) {
-      // bins from h = 1024 down: thread t sums bins 4t..4t+3 (index x = 1024 - h);
-      // bin x = 1024 (h = 0) is handled last
-      int sum = 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) sum += int(hist[1024 - (4 * tid + u)]);
-      int incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      if (lane == 31) s_wsum[warp] = incl;
-      __syncthreads();
-      int before = 0;
-      for (int w = 0; w < warp; ++w) before += s_wsum[w];
-      const int excl = before + incl - sum;
-      if (excl < R && R <= excl + sum) {
-        int run = excl;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int c = int(hist[1024 - (4 * tid + u)]);
-          if (run + c >= R) {
-            s_ht = 1024 - (4 * tid + u);
-            s_gt = run;
-            break;
-          }
-          run += c;
-        }
-      }
-      if (tid == kThreads - 1 && excl + sum < R) {  // the cut falls in bin h = 0
-        s_ht = 0;
-        s_gt = excl + sum;
-      }
-    } else if (tid == 0) {
-      s_ht = -1;  // every occurrence is selected
-      s_gt = cnt;
-    }
-    __syncthreads();
-    // ---- E  tie cut: the j of the (R - count(h > h_t))-th occurrence with h == h_t
-    //         (thread-contiguous segments keep the j order); a distinct id with
-    //         h == h_t is selected iff its first occurrence is at or before it
-    {
-      const int ht = s_ht, need_eq = R - s_gt;
-      if (ht >= 0) {
-        const int seg = (KK + kThreads - 1) / kThreads;
-        const int j0 = tid * seg, j1 = min(KK, j0 + seg);
-        int eq = 0;
-        for (int j = j0; j < j1; ++j) {
-          const int sl = cand_slot[j];
-          eq += (sl >= 0 && int((meta[sl] >> 16) & 0x7ffu) == ht) ? 1 : 0;
-        }
-        int incl = eq;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += t;
-        }
-        if (lane == 31) s_wsum2[warp] = incl;
-        __syncthreads();
-        int rank = incl - eq;
-        for (int w = 0; w < warp; ++w) rank += s_wsum2[w];
-        if (rank < need_eq && need_eq <= rank + eq) {
-          for (int j = j0; j < j1; ++j) {
-            const int sl = cand_slot[j];
-            if (sl >= 0 && int((meta[sl] >> 16) & 0x7ffu) == ht && ++rank == need_eq) {
-              s_jcut = j;
-              break;
+        for (int e = 0; e < 2; ++e) {
+          const int j = 2 * p + e;
+          if (j < LA.KK) {
+            const int k = int((uint32_t(j) * LA.kdiv) >> 20);
+            const uint32_t n1 = lds32(a_pool + 4 * k);
+            if (n1 < n) {
+              v[2 * r + e] = uint32_t(ids_in[int64_t(n1) * K + (j - k * K)]);
+              KNNG_FLAG_IF(ctl.check_err, v[2 * r + e] >= n);
             }
           }
         }
       }
     }
-    __syncthreads();
-    // ---- F1  selected distinct ids that are not starting-list members need a dot
-    {
-      const int ht = s_ht, jcut = ht >= 0 ? s_jcut : 0;
-      for (int q0 = warp * 32; q0 < nu; q0 += kThreads) {  // warp-uniform trip count
-        const int q = q0 + lane;
-        bool want = false;
-        int sl = -1;
-        if (q < nu) {
-          sl = ulist[q];
-          const uint32_t m = meta[sl];
-          const int h = int((m >> 16) & 0x7ffu);
-          const bool sel = ht < 0 || h > ht || (h == ht && int(m & kFirstMask) <= jcut);
-          // a cached rejection stands: the row's threshold never falls, so a
-          // dot once <= it stays <= it
-          want = sel && !(uint32_t(key[sl]) & kPoolFlag) && !(m & kRej);
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, want);
-        int base = 0;
-        if (lane == 0 && bal) base = atomicAdd(&s_nneed, __popc(bal));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (want) need[base + __popc(bal & ((1u << lane) - 1u))] = int16_t(sl);
-      }
+    for (int t = tid; t < (KNNG_L(pairs) * 4 + 15) / 16; t += kThreads) sts128(a_info + 16 * t, make_uint4(0, 0, 0, 0));
+    // unscored entries (INT32_MIN, tiny inputs only) can share their id with a
+    // survivor, and an unsorted pool (possible through the stage entry point)
+    // breaks the rank formulas of stage G: both take the sequential loop
+    int irregular = 0;
+    uint32_t find_id = ~0u;  // this thread's starting-list id, while it is still looked up
+    if (tid < K) {
+      const uint32_t my_id = lds32(a_pool + 4 * tid);
+      const int32_t my_sc = int32_t(lds32(a_psc + 4 * tid));
+      KNNG_FLAG_IF(ctl.check_err, my_id >= n);
+      irregular = (my_sc == kScoreMinI) | (tid + 1 < K && my_sc < int32_t(lds32(a_psc + 4 * tid + 4)));
+      if (my_sc != kScoreMinI && my_id < n) find_id = my_id;
     }
-    __syncthreads();
-    // ---- F2  dots (8 lanes per candidate, up to eight 16-byte loads in flight per lane)
-    {
-      const int nneed = s_nneed;
-      if (tid == 0) s_stat[2] += unsigned(nneed);
-      const int32_t thr0 = pool_sc[K - 1];
-      const int per_lane = d / 128;
-      for (int wbase = warp * 4; wbase < nneed; wbase += kGroups) {
-        const int q = wbase + slot8;
-        const int sl = q < nneed ? int(need[q]) : -1;
-        const int32_t id = sl >= 0 ? int32_t(uint32_t(key[sl]) & 0x7fffffffu) : 0;
-        int acc = 0;
-        if (sl >= 0) {
-          const uint4* row = reinterpret_cast<const uint4*>(codes + int64_t(id) * d);
-          uint4 v[8];
+    // a valid id goes into the first table; without a candidate the register
+    // holds kNone, which no id in shared memory equals
+    unsigned valid = 0;  // bit 2r + e
+    const uint32_t tagj = (tag << kJBits) + 2u * uint32_t(tid);
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u < per_lane) v[u] = __ldg(row + sub + 8 * u);
+    for (int r = 0; r < NP; ++r) {
+      const int p = tid + kThreads * r;
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (u < per_lane) acc = dot_u4(v[u], my_code[sub + 8 * u], acc);
+      for (int e = 0; e < 2; ++e) {
+        uint32_t& id = v[2 * r + e];
+        const bool ok = id < n && id != uint32_t(i);
+        red_min_if(ok, a_ta + slot_of(id, 0u, KNNG_L(ta_shift)), tagj + uint32_t(2 * kThreads * r + e));
+        valid |= ok ? 1u << (2 * r + e) : 0u;
+        id = ok ? id : kNone;
+      }
+      if (p < KNNG_L(pairs)) sts64(a_ids + 8 * p, v[2 * r], v[2 * r + 1]);
+    }
+    {
+      const int c = __reduce_add_sync(full, __popc(valid));
+      if (lane == 0) red_add(a_row + kRowCnt, uint32_t(c));
+    }
+    cp_async_wait_all();  // this thread's copies of stage A; the barrier publishes them
+    const bool serial_insert = __syncthreads_or(irregular) != 0;
+    unsigned fm = 0;     // bit 2r + e: the occurrence is the first of its id
+    int find_rep = -1;   // representative of the starting-list id, if it occurs
+    unsigned ctodo = 0;  // bit 2u + e: the cached id is not resolved
+    unsigned todo = 0;   // bit 2r + e: the occurrence is not resolved
+    // round 0: every occurrence, every cached id, the starting list
+    {
+      uint32_t w[2 * NP];
+#pragma unroll
+      for (int x = 0; x < 2 * NP; ++x) {
+        w[x] = lds32(a_ta + slot_of(v[x], 0u, KNNG_L(ta_shift))) & kJMask;
+        w[x] = v[x] == kNone ? KNNG_L(dummy) : w[x];
+      }
+#pragma unroll
+      for (int r = 0; r < NP; ++r) {
+        const int p = tid + kThreads * r;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const uint32_t j = uint32_t(2 * p + e), id = v[2 * r + e];
+          const bool lost = lds32(a_ids + 4 * w[2 * r + e]) != id && id != kNone;
+          red_min_if(lost, a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e));
+          todo |= lost ? 1u << (2 * r + e) : 0u;
+          fm |= w[2 * r + e] == j && p < KNNG_L(pairs) ? 1u << (2 * r + e) : 0u;
         }
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-        if (sub == 0 && sl >= 0 && acc > thr0) {
-          const uint32_t m = meta[sl];
-          const int slot = atomicAdd(&s_nprom, 1);
-          surv[slot] = make_int4(int((((m >> 16) & 0x7ffu) << 13) | (kFirstMask - (m & kFirstMask))), acc, id, 0);
-        } else if (sub == 0 && sl >= 0 && cached) {
-          meta[sl] |= kRej;
+        if (p < KNNG_L(pairs)) sts32(a_rep + 4 * p, w[2 * r] | (w[2 * r + 1] << 16));
+      }
+    }
+#pragma unroll 1
+    for (int u = 0; u < kCachePairs; ++u) {
+      if (2 * kThreads * u >= cc) break;  // block-uniform
+      const int q = tid + kThreads * u;
+      const uint2 id = lds64(a_x + 8 * q);
+      const uint32_t hr = lds32(a_hist + 4 * q);
+      const uint32_t e0 = lds32(a_ta + slot_of(id.x, 0u, KNNG_L(ta_shift)));
+      const uint32_t e1 = lds32(a_ta + slot_of(id.y, 0u, KNNG_L(ta_shift)));
+      const uint32_t w0 = e0 & kJMask, w1 = e1 & kJMask;
+      const uint32_t x0 = lds32(a_ids + 4 * w0), x1 = lds32(a_ids + 4 * w1);
+      const bool t0 = 2 * q < cc && (e0 >> kJBits) == tag, t1 = 2 * q + 1 < cc && (e1 >> kJBits) == tag;
+      sts16_if(t0 && x0 == id.x, a_info + 2 * w0, hr | kKnown);
+      sts16_if(t1 && x1 == id.y, a_info + 2 * w1, (hr >> 16) | kKnown);
+      ctodo |= (t0 && x0 != id.x ? 1u << (2 * u) : 0u) | (t1 && x1 != id.y ? 2u << (2 * u) : 0u);
+    }
+    if (find_id != ~0u) {
+      const uint32_t e = lds32(a_ta + slot_of(find_id, 0u, KNNG_L(ta_shift)));
+      if ((e >> kJBits) != tag) {
+        find_id = ~0u;
+      } else if (lds32(a_ids + 4 * (e & kJMask)) == find_id) {
+        find_rep = int(e & kJMask);
+        find_id = ~0u;
+      }
+    }
+    uint32_t round = 1;
+#pragma unroll 1
+    while (__syncthreads_or(int(todo))) {
+      const bool odd = round & 1u;
+      const uint32_t t_cur = odd ? a_tb : a_ta, t_nxt = odd ? a_ta : a_tb;
+      const int sh_cur = odd ? kTableBShift : KNNG_L(ta_shift), sh_nxt = odd ? KNNG_L(ta_shift) : kTableBShift;
+      const uint32_t tc = tag - round;
+#pragma unroll 1
+      for (unsigned m = todo; m; m &= m - 1u) {
+        const int b = __ffs(m) - 1;
+        const uint32_t j = 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1);
+        const uint32_t id = lds32(a_ids + 4 * j);
+        const uint32_t w = lds32(t_cur + slot_of(id, round, sh_cur)) & kJMask;
+        if (lds32(a_ids + 4 * w) == id) {
+          sts16(a_rep + 2 * j, w);
+          todo ^= 1u << b;
+          if (w == j) fm |= 1u << b;
+        } else {
+          red_min(t_nxt + slot_of(id, round + 1u, sh_nxt), ((tc - 1u) << kJBits) + j);
         }
+      }
+#pragma unroll 1
+      for (unsigned m = ctodo; m; m &= m - 1u) {
+        const int b = __ffs(m) - 1;
+        const uint32_t q = 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1);
+        const uint32_t id = lds32(a_x + 4 * q);
+        const uint32_t e = lds32(t_cur + slot_of(id, round, sh_cur));
+        if ((e >> kJBits) != tc) {
+          ctodo ^= 1u << b;
+        } else if (lds32(a_ids + 4 * (e & kJMask)) == id) {
+          ctodo ^= 1u << b;
+          sts16(a_info + 2 * (e & kJMask), lds16(a_hist + 2 * q) | kKnown);
+        }
+      }
+      if (find_id != ~0u) {
+        const uint32_t e = lds32(t_cur + slot_of(find_id, round, sh_cur));
+        if ((e >> kJBits) != tc) {
+          find_id = ~0u;
+        } else if (lds32(a_ids + 4 * (e & kJMask)) == find_id) {
+          find_rep = int(e & kJMask);
+          find_id = ~0u;
+        }
+      }
+      ++round;
+    }
+    tag -= round + 1u;
+    fetch_list(slot ^ 1u);  // the previous row's list is no longer read
+    // ---- C  Hamming once per distinct id without a cached distance: each warp
+    //         lists its own first occurrences that are misses and scores them
+    //         (groups of 8 lanes, CB candidates in flight per group)
+    if (find_rep >= 0) sts32(a_ids + 4 * find_rep, lds32(a_ids + 4 * find_rep) | kPoolFlag);
+    for (int t = tid; t < kHBins / 4; t += kThreads) sts128(a_hist + 16 * t, make_uint4(0, 0, 0, 0));
+    int first_at;  // this thread's place among the row's distinct ids (stage G)
+    {
+      unsigned mm = fm;
+      if (cc > 0) {  // block-uniform
+#pragma unroll
+        for (int r = 0; r < NP; ++r) {
+          const int p = tid + kThreads * r;
+          if (p < KNNG_L(pairs)) {
+            const uint32_t f = lds32(a_info + 4 * p);
+            if (f & kKnown) mm &= ~(1u << (2 * r));
+            if (f & (kKnown << 16)) mm &= ~(2u << (2 * r));
+          }
+        }
+      }
+      const int c = __popc(mm), incl = warp_incl_scan(c, lane);
+      const int nm = __shfl_sync(full, incl, 31);
+      const int nfirst = __popc(fm), fincl = warp_incl_scan(nfirst, lane);
+      int wbase = 0;
+      if (lane == 31) {
+        wbase = int(atom_add(a_row + kRowNu, uint32_t(fincl)));
+        red_add(a_row + kRowMiss, uint32_t(incl));
+      }
+      first_at = __shfl_sync(full, wbase, 31) + fincl - nfirst;
+      // up to 64 NP misses per warp
+      const uint32_t a_miss = a_x + uint32_t(warp) * (DEF ? uint32_t(NP) * 128u : uint32_t((LA.pairs + kThreads - 1) / kThreads) * 128u);
+      uint32_t at = a_miss + 2 * (incl - c);
+#pragma unroll 1
+      for (; mm; mm &= mm - 1u, at += 2) {
+        const int b = __ffs(mm) - 1;
+        sts16(at, 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1));
+      }
+      __syncwarp();
+      const char* sk_base = reinterpret_cast<const char*>(sketch);
+      const uint32_t sk_bytes = uint32_t(W) * 8u;
+      if (sk_chunks == 1) {  // 16-byte sketches: one lane per candidate
+        const uint4 mine = lds128(sb + KNNG_L(o_sk));
+#pragma unroll 1
+        for (int q = lane; q < nm; q += 32) {
+          const uint32_t j = lds16(a_miss + 2 * q), id = lds32(a_ids + 4 * j) & ~kPoolFlag;
+          sts16(a_info + 2 * j, popc_u4(__ldg(reinterpret_cast<const uint4*>(sk_base + uint64_t(id) * 16u)), mine));
+        }
+      } else {
+        // 32 candidates per step, 8 lanes each: lane 8g + s reads the 16-byte
+        // chunk s of candidates 4u + g (u = 0..7) and ends up with the
+        // distance of candidate 4 t(s) + g, where t reverses s's three bits:
+        // the group's 8 partial sums are two to a word, and each exchange
+        // keeps half of the words (14 instructions for 8 sums, against 48
+        // for one butterfly per sum)
+        const uint4 mine = sub < sk_chunks ? lds128(sb + KNNG_L(o_sk) + 16 * sub) : make_uint4(0, 0, 0, 0);
+        const char* sk_lane = sk_base + 16 * (sub < sk_chunks ? sub : 0);
+        const int t = ((sub & 1) << 2) | (sub & 2) | (sub >> 2);
+#pragma unroll 1
+        for (int b = 0; b < nm; b += 32) {
+          const int q = b + 4 * t + slot8;
+          uint32_t j = 0, id = uint32_t(i);  // past the list: the row itself
+          if (q < nm) {
+            j = lds16(a_miss + 2 * q);
+            id = lds32(a_ids + 4 * j) & ~kPoolFlag;
+          }
+          uint32_t pw[4] = {0, 0, 0, 0};  // word k: candidates u = k (low half) and u = k + 4
+#pragma unroll
+          for (int u0 = 0; u0 < 8; u0 += CB) {
+            if (b + 4 * u0 >= nm) break;  // warp-uniform
+            uint4 x[CB];
+#pragma unroll
+            for (int u = 0; u < CB; ++u) {
+              const int uu = u0 + u, src = ((uu & 1) << 2) | (uu & 2) | (uu >> 2);  // the lane whose t is uu
+              const uint32_t cid = __shfl_sync(full, id, 8 * slot8 + src);
+              x[u] = __ldg(reinterpret_cast<const uint4*>(sk_lane + uint64_t(cid) * sk_bytes));
+            }
+#pragma unroll
+            for (int u = 0; u < CB; ++u) {
+              const uint32_t pc = popc_u4(x[u], mine);
+              pw[(u0 + u) & 3] += (u0 + u) < 4 ? pc : pc << 16;
+            }
+          }
+          if (sub >= sk_chunks) pw[0] = pw[1] = pw[2] = pw[3] = 0;  // lanes beyond a narrow sketch
+          // exchange 1 (lane bit 0 = bit 2 of t): nothing to choose between, both
+          // halves of a word stay together; it is left for the last step.
+          // Lane bit 1 is bit 1 of t (word pairs 0,1 / 2,3), lane bit 2 bit 0.
+          const bool s1 = sub & 2, s2 = sub & 4;
+          uint32_t k0 = s1 ? pw[2] : pw[0], k1 = s1 ? pw[3] : pw[1];
+          k0 += __shfl_xor_sync(full, s1 ? pw[0] : pw[2], 2);
+          k1 += __shfl_xor_sync(full, s1 ? pw[1] : pw[3], 2);
+          uint32_t k = s2 ? k1 : k0;
+          k += __shfl_xor_sync(full, s2 ? k0 : k1, 4);
+          k += __shfl_xor_sync(full, k, 1);
+          if (q < nm) sts16(a_info + 2 * j, (sub & 1) ? k >> 16 : k & 0xffffu);
+        }
+      }
+    }
+    fetch_flags(slot ^ 1u);
+    __syncthreads();
+    // ---- D  histogram over occurrences, threshold
+    uint32_t hv[NP];  // info of each occurrence's id, two per word
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+      const int p = tid + kThreads * r;
+      hv[r] = kNoDist | (kNoDist << 16);
+      if (p < KNNG_L(pairs)) {
+        const uint32_t w = lds32(a_rep + 4 * p);
+        const uint32_t f0 = lds16(a_info + 2 * (w & 0xffffu)), f1 = lds16(a_info + 2 * (w >> 16));
+        hv[r] = f0 | (f1 << 16);
+        red_add(a_hist + 4 * (f0 & kXMask), 1u);
+        red_add(a_hist + 4 * (f1 & kXMask), 1u);
       }
     }
     __syncthreads();
-    // ---- F3  the row's cache for the next iteration: this iteration's distinct
-    //          candidates (the first cache_cap of them) with score and flag
-    if (cached) {
-      const int cc = min(nu, ctl.cache_cap);
-      int32_t* cid = ctl.cache_ids + i * ctl.cache_cap;
-      uint16_t* chr = ctl.cache_hr + i * ctl.cache_cap;
-      for (int q = tid; q < cc; q += kThreads) {
-        const int sl = ulist[q];
-        const uint32_t m = meta[sl];
-        cid[q] = int32_t(uint32_t(key[sl]) & 0x7fffffffu);
-        chr[q] = uint16_t((((m >> 16) & 0x7ffu) << 1) | ((m & kRej) ? 1u : 0u));
+    uint32_t xt = kXMask;  // threshold distance; none: every occurrence is nearer
+    int need_eq = 0;
+    const bool cut = int(lds32(a_row + kRowCnt)) > R;  // block-uniform
+    if (cut) {
+      // every warp by itself: bins from distance 0 up, 128 per step
+      int acc = 0;
+#pragma unroll 1
+      for (int base = 0; base < kHBins; base += 128) {
+        const uint4 b4 = lds128(a_hist + 4 * (base + 4 * lane));
+        const int sum = int(b4.x + b4.y + b4.z + b4.w), incl = warp_incl_scan(sum, lane);
+        const int tot = __shfl_sync(full, incl, 31);
+        if (acc + tot >= R) {  // warp-uniform; reached, as the bins hold cnt > R occurrences
+          int run = acc + incl - sum, x = base + 4 * lane;
+          const bool here = run < R && R <= run + sum;
+          if (run + int(b4.x) < R) {
+            run += int(b4.x);
+            ++x;
+            if (run + int(b4.y) < R) {
+              run += int(b4.y);
+              ++x;
+              if (run + int(b4.z) < R) {
+                run += int(b4.z);
+                ++x;
+              }
+            }
+          }
+          const int src = __ffs(__ballot_sync(full, here)) - 1;
+          xt = uint32_t(__shfl_sync(full, x, src));
+          need_eq = R - __shfl_sync(full, run, src);
+          break;
+        }
+        acc += tot;
       }
-      if (tid == 0) ctl.cache_cnt[i] = cc;
     }
-    // ---- G/H  insertion of the survivors in visit order (pkey descending;
-    //   keys are distinct).  The new pool goes to new_id/new_sc, laid over the
-    //   hash table, which is dead after F2.
-    const int P = s_nprom;
-    int32_t* new_id = reinterpret_cast<int32_t*>(hist);  // dead after stage E; stage F3 may still read the table
-    int32_t* new_sc = new_id + kMaxK;
-    if (!serial_insert) {
-      // The pool's last score only rises during the visits, and a rejected
-      // survivor's dot is <= the last score at its visit, so the last score
-      // before visit t is the K-th largest of {starting scores} and {dots of
-      // all survivors visited before t}: survivor t is inserted iff fewer
-      // than K of those values are >= its dot.  The final pool is the best K of
-      // (starting entries, inserted survivors) ordered by score, ties to the
-      // starting entries (in pool order) and then to earlier visits -- the
-      // order the shift-insert loop leaves.  Needs a sorted starting pool
-      // without unscored entries (else serial_insert is set).
-      // A survivor record is {visit key, dot, id, flags}; flags bit 31 =
-      // inserted, bits 0..30 = starting scores >= dot.  Stage G1 reads only
-      // the first two words of the other records, so writing a record's
-      // flags word does not race with it.
-      for (int p = tid; p < P; p += kThreads) {
-        const int2 me = *reinterpret_cast<const int2*>(surv + p);
-        const uint32_t kp = uint32_t(me.x);
-        const int32_t dp = me.y;
-        int lo = 0, hi = K;  // first pool position with a score < dp (scores descend)
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (pool_sc[mid] >= dp) lo = mid + 1;
-          else hi = mid;
+    // ---- E  selected first occurrences that are neither starting-list members
+    //         nor known to be rejected need a dot; one at the threshold is
+    //         selected iff fewer than need_eq ties come before it in j order
+    //         (a cached rejection stands: the row's threshold never falls, so
+    //         a dot once <= it stays <= it)
+    unsigned wm = 0, eqm = 0;  // nearer than the threshold; at it
+#pragma unroll
+    for (int r = 0; r < NP; ++r) {
+      const uint32_t x0 = hv[r] & kXMask, x1 = (hv[r] >> 16) & kXMask;
+      if (x0 < xt && !(hv[r] & kRej)) wm |= 1u << (2 * r);
+      if (x1 < xt && !(hv[r] & (kRej << 16))) wm |= 2u << (2 * r);
+      if (x0 == xt) eqm |= 1u << (2 * r);
+      if (x1 == xt) eqm |= 2u << (2 * r);
+    }
+    wm &= fm;
+    if (cut) {
+      // ties per (round, warp): j ascends with round, warp, lane, element
+      const unsigned any = __reduce_or_sync(full, eqm);
+#pragma unroll
+      for (int r = 0; r < NP; ++r) {
+        int c = 0;
+        if ((any >> (2 * r)) & 3u) {  // warp-uniform
+          c = __popc(__ballot_sync(full, (eqm >> (2 * r)) & 1u)) + __popc(__ballot_sync(full, (eqm >> (2 * r)) & 2u));
         }
-        int c = lo;
-#pragma unroll 4
-        for (int q = 0; q < P; ++q) {
-          const int2 o = *reinterpret_cast<const int2*>(surv + q);
-          c += (uint32_t(o.x) > kp && o.y >= dp) ? 1 : 0;
-        }
-        surv[p].w = int(uint32_t(lo) | (c < K ? 0x80000000u : 0u));
+        if (lane == 0) sts32(a_cell + 4 * (r * kWarps + warp), uint32_t(c));
       }
       __syncthreads();
-      // one unit per thread: starting entries 0..K-1, then survivors
-      for (int u = tid; u < K + P; u += kThreads) {
-        if (u < K) {
-          const int32_t s = pool_sc[u];
-          int rank = u;
-#pragma unroll 4
-          for (int q = 0; q < P; ++q) {
-            const int4 o = surv[q];
-            rank += (o.w < 0 && o.y > s) ? 1 : 0;
-          }
-          if (rank < K) {
-            new_id[rank] = pool_id[u];
-            new_sc[rank] = s;
-          }
-        } else {
-          const int4 me = surv[u - K];
-          if (me.w >= 0) continue;  // not inserted
-          int rank = me.w & 0x7fffffff;
-#pragma unroll 4
-          for (int q = 0; q < P; ++q) {
-            const int4 o = surv[q];
-            rank += (o.w < 0 && (o.y > me.y || (o.y == me.y && uint32_t(o.x) > uint32_t(me.x)))) ? 1 : 0;
-          }
-          if (rank < K) {
-            new_id[rank] = me.z;
-            new_sc[rank] = me.y;
+      if (any) {  // warp-uniform
+        uint2 c2 = make_uint2(0, 0);
+        if (2 * lane < NP * kWarps) c2 = lds64(a_cell + 8 * lane);
+        const int sum = int(c2.x + c2.y);
+        const int pre = warp_incl_scan(sum, lane) - sum + ((warp & 1) ? int(c2.x) : 0);
+#pragma unroll
+        for (int r = 0; r < NP; ++r) {
+          if ((any >> (2 * r)) & 3u) {  // warp-uniform
+            const unsigned b0 = __ballot_sync(full, (eqm >> (2 * r)) & 1u), b1 = __ballot_sync(full, (eqm >> (2 * r)) & 2u);
+            const int before = __shfl_sync(full, pre, 4 * r + (warp >> 1)) + __popc(b0 & lt) + __popc(b1 & lt);
+            const unsigned e0 = (eqm >> (2 * r)) & 1u;
+            if (e0 && before < need_eq && !(hv[r] & kRej)) wm |= (1u << (2 * r)) & fm;
+            if (((eqm >> (2 * r)) & 2u) && before + int(e0) < need_eq && !(hv[r] & (kRej << 16))) wm |= (2u << (2 * r)) & fm;
           }
         }
       }
-    } else {
-    // rank sort by (h desc, first j asc), then the reference's shift-insert
-    // loop in warp 0 with the pool held two entries per lane
-    for (int p = tid; p < P; p += kThreads) {
-      const uint32_t kp = uint32_t(surv[p].x);
-      int rank = 0;
-      for (int q = 0; q < P; ++q) rank += uint32_t(surv[q].x) > kp ? 1 : 0;
-      order[rank] = uint16_t(p);
+    }
+    {
+#pragma unroll 1
+      for (unsigned m = wm; m; m &= m - 1u) {
+        const int b = __ffs(m) - 1;
+        if (int32_t(lds32(a_ids + 8 * (tid + kThreads * (b >> 1)) + 4 * (b & 1))) < 0) wm ^= 1u << b;
+      }
+      if (__any_sync(full, wm != 0)) {
+        const int c = __popc(wm), incl = warp_incl_scan(c, lane);
+        uint32_t base = 0;
+        if (lane == 31) base = atom_add(a_row + kRowNeed, uint32_t(incl));
+        uint32_t at = a_x + 2 * (__shfl_sync(full, base, 31) + uint32_t(incl - c));
+#pragma unroll 1
+        for (; wm; wm &= wm - 1u, at += 2) {
+          const int b = __ffs(wm) - 1;
+          sts16(at, 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1));
+        }
+      }
     }
     __syncthreads();
-    if (warp == 0) {
-      int32_t idA = lane < K ? pool_id[lane] : -1, scA = lane < K ? pool_sc[lane] : kScoreMinI;
-      int32_t idB = 32 + lane < K ? pool_id[32 + lane] : -1, scB = 32 + lane < K ? pool_sc[32 + lane] : kScoreMinI;
-      const unsigned full = 0xffffffffu;
-      for (int rr = 0; rr < P; ++rr) {
-        const int p = order[rr];
-        const int32_t id = surv[p].z, dot = surv[p].y;
-        if (__any_sync(full, idA == id || idB == id)) continue;
-        const int32_t last = (K - 1) < 32 ? __shfl_sync(full, scA, K - 1) : __shfl_sync(full, scB, K - 33);
-        if (!(dot > last)) continue;
-        const int pos = __popc(__ballot_sync(full, lane < K - 1 && scA >= dot)) +
-                        __popc(__ballot_sync(full, 32 + lane < K - 1 && scB >= dot));
-        const int32_t upIdA = __shfl_up_sync(full, idA, 1), upScA = __shfl_up_sync(full, scA, 1);
-        const int32_t upIdB = __shfl_up_sync(full, idB, 1), upScB = __shfl_up_sync(full, scB, 1);
-        const int32_t id31 = __shfl_sync(full, idA, 31), sc31 = __shfl_sync(full, scA, 31);
-        if (lane < K) {
-          if (lane > pos) { idA = upIdA; scA = upScA; }
-          else if (lane == pos) { idA = id; scA = dot; }
+    // ---- F  dots (8 lanes per candidate, up to eight 16-byte loads in flight per lane)
+    {
+      const int per_lane = d / 128;
+#pragma unroll 1
+      for (int q = warp * 4 + slot8; q - slot8 < int(lds32(a_row + kRowNeed)); q += kGroups) {
+        const bool live = q < int(lds32(a_row + kRowNeed));
+        int acc = 0;
+        if (live) {
+          const uint32_t id = lds32(a_ids + 4 * lds16(a_x + 2 * q));
+          const int8_t* row = codes + int64_t(id) * d + 16 * sub;
+          const uint32_t mine = a_code + 16 * sub;
+          switch (per_lane) {  // uniform; one body per width, so that all its loads are in flight without predicates
+            case 1: acc = dot_lane<1>(row, mine); break;
+            case 2: acc = dot_lane<2>(row, mine); break;
+            case 3: acc = dot_lane<3>(row, mine); break;
+            case 4: acc = dot_lane<4>(row, mine); break;
+            case 5: acc = dot_lane<5>(row, mine); break;
+            case 6: acc = dot_lane<6>(row, mine); break;
+            case 7: acc = dot_lane<7>(row, mine); break;
+            default: acc = dot_lane<8>(row, mine); break;
+          }
         }
-        const int qb = 32 + lane;
-        if (qb < K) {
-          if (qb > pos) {
-            idB = lane == 0 ? id31 : upIdB;
-            scB = lane == 0 ? sc31 : upScB;
-          } else if (qb == pos) {
-            idB = id;
-            scB = dot;
+        acc += __shfl_xor_sync(full, acc, 1);
+        acc += __shfl_xor_sync(full, acc, 2);
+        acc += __shfl_xor_sync(full, acc, 4);
+        if (sub == 0 && live) {
+          const uint32_t j = lds16(a_x + 2 * q), id = lds32(a_ids + 4 * j), f = lds16(a_info + 2 * j);
+          if (acc > int32_t(lds32(a_psc + 4 * (K - 1)))) {
+            const uint32_t at = atom_add(a_row + kRowProm, 1u);
+            sts64(a_rep + 8 * at, ((1024u - (f & kXMask)) << 13) | (0x1fffu - j), uint32_t(acc) ^ 0x80000000u);
+            sts32(a_sid + 4 * at, id);
+          } else if (cached) {
+            sts16(a_info + 2 * j, f | kRej);
           }
         }
       }
-      if (lane < K) {
-        new_id[lane] = idA;
-        new_sc[lane] = scA;
-      }
-      if (32 + lane < K) {
-        new_id[32 + lane] = idB;
-        new_sc[32 + lane] = scB;
-      }
-    }
     }
     __syncthreads();
-    // ---- write-back of the positions whose id changed (every position when
-    //      the output is the other buffer) and the update count
-    if (warp == 0) {
-      const unsigned full = 0xffffffffu;
+    // ---- G  the row's cache for the next iteration: this iteration's distinct
+    //         candidates (the first cache_cap of them) with distance and flag,
+    //         gathered in shared memory (over the rerank list and the
+    //         histogram) and written out 16 bytes at a time below
+    if (cached) {
+#pragma unroll 1
+      for (unsigned m = fm; m; m &= m - 1u, ++first_at) {
+        if (first_at >= ctl.cache_cap) break;
+        const int b = __ffs(m) - 1;
+        const uint32_t j = 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1);
+        const uint32_t id = lds32(a_ids + 4 * j), f = lds16(a_info + 2 * j);
+        sts32(a_x + 4 * first_at, id & ~kPoolFlag);
+        sts16(a_hist + 2 * first_at, f & ~kKnown);
+      }
+    }
+    //         insertion of the survivors in visit order.  The pool's last score
+    //         only rises during the visits, and a rejected survivor's dot is <=
+    //         the last score at its visit, so survivor t is rejected iff at
+    //         least K of {starting scores} and {dots of the survivors visited
+    //         before t} are >= its dot: iff K entries come before it in the
+    //         order (score desc, starting entries in pool order first, then
+    //         earlier visits).  The final pool, which the shift-insert loop
+    //         leaves in that order, is therefore the first K of the starting
+    //         entries and all survivors.  Needs a sorted starting pool without
+    //         unscored entries (else serial_insert is set).
+    const int P = int(lds32(a_row + kRowProm));
+    int32_t* out_id = ids_out + int64_t(i) * K;
+    int32_t* out_sc = scores_out + int64_t(i) * K;
+    if (P == 0) {  // block-uniform: the list stays
+      if (!inplace && tid < K) {
+        out_id[tid] = int32_t(lds32(a_pool + 4 * tid));
+        out_sc[tid] = int32_t(lds32(a_psc + 4 * tid));
+      }
+    } else if (!serial_insert) {
       int changed = 0;
-      for (int k = lane; k < K; k += 32) {
-        const int32_t nid = new_id[k];
-        const bool ch = nid != pool_id[k];
-        changed += ch;
-        if (ch || !inplace) {
-          ids_out[i * K + k] = nid;
-          scores_out[i * K + k] = new_sc[k];
+      // one unit per thread: starting entries 0..K-1, then survivors
+#pragma unroll 1
+      for (int u = tid; u < K + P; u += kThreads) {
+        uint64_t me;
+        uint32_t id;
+        int rank;
+        if (u < K) {
+          // survivors with a larger dot come first: their keys are above (score, all ones)
+          me = (uint64_t(lds32(a_psc + 4 * u) ^ 0x80000000u) << 32) | 0xffffffffu;
+          id = lds32(a_pool + 4 * u);
+          rank = u;
+        } else {
+          const uint2 k2 = lds64(a_rep + 8 * (u - K));
+          me = (uint64_t(k2.y) << 32) | k2.x;
+          id = lds32(a_sid + 4 * (u - K));
+          const int32_t dot = int32_t(k2.y ^ 0x80000000u);
+          int lo = 0, hi = K;  // first pool position with a score < dot (scores descend)
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (int32_t(lds32(a_psc + 4 * mid)) >= dot) lo = mid + 1;
+            else hi = mid;
+          }
+          rank = lo;
+        }
+        int q = 0;
+#pragma unroll 2
+        for (; q + 1 < P; q += 2) {
+          const uint4 o = lds128(a_rep + 8 * q);
+          rank += ((uint64_t(o.y) << 32) | o.x) > me ? 1 : 0;
+          rank += ((uint64_t(o.w) << 32) | o.z) > me ? 1 : 0;
+        }
+        if (q < P) {
+          const uint2 o = lds64(a_rep + 8 * q);
+          rank += ((uint64_t(o.y) << 32) | o.x) > me ? 1 : 0;
+        }
+        if (rank < K) {
+          const bool ch = id != lds32(a_pool + 4 * rank);
+          changed += ch ? 1 : 0;
+          if (ch || !inplace) {
+            out_id[rank] = int32_t(id);
+            out_sc[rank] = int32_t(uint32_t(me >> 32) ^ 0x80000000u);
+          }
         }
       }
-      for (int o = 16; o > 0; o >>= 1) changed += __shfl_xor_sync(full, changed, o);
-      if (lane == 0) s_stat[0] += unsigned(changed);
-      if (ctl.chg_out && lane == 0) ctl.chg_out[i] = changed ? 1 : 0;
-      if (ctl.job_upd && lane == 0) {
-        if (job != run_job) {
-          if (run_job >= 0 && run_upd) atomicAdd(ctl.job_upd + run_job, run_upd);
-          run_job = job;
-          run_upd = 0;
+      changed = __reduce_add_sync(full, changed);
+      if (lane == 0 && changed) red_add(a_row + kRowChanged, uint32_t(changed));
+    } else {
+      // rank sort by (h desc, first j asc), then the reference's shift-insert
+      // loop in warp 0 with the pool held two entries per lane
+#pragma unroll 1
+      for (int p = tid; p < P; p += kThreads) {
+        const uint32_t kp = lds32(a_rep + 8 * p);
+        int rank = 0;
+        for (int q = 0; q < P; ++q) rank += lds32(a_rep + 8 * q) > kp ? 1 : 0;
+        sts16(a_sorder + 2 * rank, uint32_t(p));
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const int32_t pidA = lane < K ? int32_t(lds32(a_pool + 4 * lane)) : -1;
+        const int32_t pidB = 32 + lane < K ? int32_t(lds32(a_pool + 4 * (32 + lane))) : -1;
+        int32_t idA = pidA, scA = lane < K ? int32_t(lds32(a_psc + 4 * lane)) : kScoreMinI;
+        int32_t idB = pidB, scB = 32 + lane < K ? int32_t(lds32(a_psc + 4 * (32 + lane))) : kScoreMinI;
+#pragma unroll 1
+        for (int rr = 0; rr < P; ++rr) {
+          const uint32_t p = lds16(a_sorder + 2 * rr);
+          const int32_t id = int32_t(lds32(a_sid + 4 * p)), dot = int32_t(lds32(a_rep + 8 * p + 4) ^ 0x80000000u);
+          if (__any_sync(full, idA == id || idB == id)) continue;
+          const int32_t last = (K - 1) < 32 ? __shfl_sync(full, scA, K - 1) : __shfl_sync(full, scB, K - 33);
+          if (!(dot > last)) continue;
+          const int pos = __popc(__ballot_sync(full, lane < K - 1 && scA >= dot)) +
+                          __popc(__ballot_sync(full, 32 + lane < K - 1 && scB >= dot));
+          const int32_t upIdA = __shfl_up_sync(full, idA, 1), upScA = __shfl_up_sync(full, scA, 1);
+          const int32_t upIdB = __shfl_up_sync(full, idB, 1), upScB = __shfl_up_sync(full, scB, 1);
+          const int32_t id31 = __shfl_sync(full, idA, 31), sc31 = __shfl_sync(full, scA, 31);
+          if (lane < K) {
+            if (lane > pos) { idA = upIdA; scA = upScA; }
+            else if (lane == pos) { idA = id; scA = dot; }
+          }
+          const int qb = 32 + lane;
+          if (qb < K) {
+            if (qb > pos) {
+              idB = lane == 0 ? id31 : upIdB;
+              scB = lane == 0 ? sc31 : upScB;
+            } else if (qb == pos) {
+              idB = id;
+              scB = dot;
+            }
+          }
         }
-        run_upd += unsigned(changed);
+        const bool chA = lane < K && idA != pidA, chB = 32 + lane < K && idB != pidB;
+        if (lane < K && (chA || !inplace)) {
+          out_id[lane] = idA;
+          out_sc[lane] = scA;
+        }
+        if (32 + lane < K && (chB || !inplace)) {
+          out_id[32 + lane] = idB;
+          out_sc[32 + lane] = scB;
+        }
+        const int changed = __popc(__ballot_sync(full, chA)) + __popc(__ballot_sync(full, chB));
+        if (lane == 0) sts32(a_row + kRowChanged, uint32_t(changed));
       }
     }
-    __syncthreads();
+    if (cached) {
+      __syncthreads();
+      const int nc = min(int(lds32(a_row + kRowNu)), ctl.cache_cap);
+      uint4* cid = reinterpret_cast<uint4*>(ctl.cache_ids + int64_t(i) * ctl.cache_cap);
+      uint4* chr = reinterpret_cast<uint4*>(ctl.cache_hr + int64_t(i) * ctl.cache_cap);
+      const int n_id = (nc * 4 + 15) / 16, n_hr = (nc * 2 + 15) / 16;  // the last words' ends are never read
+      for (int t = tid; t < n_id; t += kThreads) cid[t] = lds128(a_x + 16 * t);
+      for (int t = tid; t < n_hr; t += kThreads) chr[t] = lds128(a_hist + 16 * t);
+      if (tid == 0) ctl.cache_cnt[i] = nc;
+    }
+    if (tid == 0) {
+      s_pend_i = i;
+      s_pend_job = s_job[slot];
+    }
+    par ^= 1u;
   }
+  __syncthreads();
+  finish_row();
   if (tid == 0) {
     atomicAdd(counters + 0, s_stat[0]);
     atomicAdd(counters + 1, s_stat[1]);
     atomicAdd(counters + 2, s_stat[2]);
     atomicAdd(counters + 3, s_stat[3]);
     if (ctl.chg_in) atomicAdd(counters + 4, s_stat[4]);
-    if (ctl.job_upd && run_job >= 0 && run_upd) atomicAdd(ctl.job_upd + run_job, run_upd);
+    if (ctl.job_upd && s_run_job >= 0 && s_run_upd) atomicAdd(ctl.job_upd + s_run_job, s_run_upd);
   }
+#undef KNNG_L
 }
 
 // Per-job early stop after an iteration, src/main.cpp:432-439 in float
@@ -764,52 +1078,64 @@ __global__ void stop_check_kernel(JobTable jt, JoinCtl ctl, int K, int iter, int
 
 }  // namespace
 
-size_t join_smem_bytes(int K, int R, int d) { return join_smem(K, R, d).bytes; }
-
 // Resident CTAs per SM of a join variant at `smem` bytes of dynamic shared
 // memory.  The attribute is set and the occupancy queried once per process and
 // variant (under a mutex, so concurrent contexts and stream captures never
 // issue these calls); a failure is returned as a CUDA error, not masked.
 std::mutex g_variant_mu;
-std::map<std::tuple<int, int, size_t>, int> g_variant_ctas;
+std::map<std::pair<const void*, uint32_t>, int> g_variant_ctas;
 char g_variant_err[256] = "";
 
-template <int CB, int MINB>
-cudaError_t max_ctas(size_t smem, int* per_sm_out) {
+using JoinKernel = void (*)(const int8_t*, const uint64_t*, int64_t, int, int, int, int, const int32_t*, const int32_t*,
+                            int32_t*, int32_t*, const int32_t*, unsigned long long*, JobTable, JoinCtl, JoinLayout);
+
+// ctas_per_sm 3: up to 80 registers per thread, 3 resident CTAs; otherwise 64
+// registers, 4 resident CTAs.
+template <bool DEF>
+JoinKernel pick_variant(int ctas_per_sm, int cblock) {
+  if (ctas_per_sm == 3)
+    return cblock == 2 ? join_kernel<2, 3, DEF> : cblock == 8 ? join_kernel<8, 3, DEF> : join_kernel<4, 3, DEF>;
+  return cblock == 2 ? join_kernel<2, 4, DEF> : cblock == 8 ? join_kernel<8, 4, DEF> : join_kernel<4, 4, DEF>;
+}
+// The kernel and shared-memory layout of a launch: the default K and R have
+// their own kernel, which reads the lists 8 bytes at a time (`aligned`).
+JoinKernel variant(int K, int R, int d, bool aligned, int ctas_per_sm, int cblock, JoinLayout* L) {
+  const bool def = K == kDefK && R == kDefR && aligned;
+  *L = join_layout(K, R, def ? kMaxDim : d);
+  return def ? pick_variant<true>(ctas_per_sm, cblock) : pick_variant<false>(ctas_per_sm, cblock);
+}
+
+cudaError_t max_ctas(JoinKernel kern, int ctas_per_sm, int cblock, uint32_t smem, int* per_sm_out) {
   std::lock_guard<std::mutex> lk(g_variant_mu);
-  const auto key = std::make_tuple(CB, MINB, smem);
+  const void* func = reinterpret_cast<const void*>(kern);
+  const auto key = std::make_pair(func, smem);
   auto it = g_variant_ctas.find(key);
   if (it != g_variant_ctas.end()) {
     *per_sm_out = it->second;
     return cudaSuccess;
   }
   cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, join_kernel<CB, MINB>);  // loads the function
+  cudaError_t e = cudaFuncGetAttributes(&fa, func);  // loads the function
   const char* what = "cudaFuncGetAttributes";
   if (e == cudaSuccess) {
-    e = ensure_smem_attr(reinterpret_cast<const void*>(join_kernel<CB, MINB>), smem);
+    e = ensure_smem_attr(func, smem);
     what = "cudaFuncSetAttribute";
   }
   int per_sm = 0;
   if (e == cudaSuccess) {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, join_kernel<CB, MINB>, kThreads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, kThreads, smem);
     what = "cudaOccupancyMaxActiveBlocksPerMultiprocessor";
   }
   if (e != cudaSuccess) {
     cudaGetLastError();  // reported through the return value
-    std::snprintf(g_variant_err, sizeof(g_variant_err), "%s(join_kernel<%d,%d>, smem %zu, static smem %zu, regs %d): %s",
-                  what, CB, MINB, smem, size_t(fa.sharedSizeBytes), fa.numRegs, cudaGetErrorString(e));
+    std::snprintf(g_variant_err, sizeof(g_variant_err), "%s(join_kernel<%d,%d>, smem %u, static smem %zu, regs %d): %s",
+                  what, cblock, ctas_per_sm, smem, size_t(fa.sharedSizeBytes), fa.numRegs, cudaGetErrorString(e));
     return e;
   }
   per_sm = per_sm < 1 ? 1 : per_sm;
   g_variant_ctas.emplace(key, per_sm);
   *per_sm_out = per_sm;
   return cudaSuccess;
-}
-
-int join_max_ctas_per_sm(int K, int R, int d) {
-  int per_sm = 1;
-  return max_ctas<4, 4>(join_smem(K, R, d).bytes, &per_sm) == cudaSuccess ? per_sm : 1;
 }
 
 const char* join_variant_error() { return g_variant_err; }
@@ -824,16 +1150,10 @@ cudaError_t join_prepare_all(int K, int R, int d) {
 }
 
 cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock) {
-  const size_t smem = join_smem(K, R, d).bytes;
+  JoinLayout L;
   int per_sm = 0;
-  if (ctas_per_sm == 3) {
-    if (cblock == 2) return max_ctas<2, 3>(smem, &per_sm);
-    if (cblock == 8) return max_ctas<8, 3>(smem, &per_sm);
-    return max_ctas<4, 3>(smem, &per_sm);
-  }
-  if (cblock == 2) return max_ctas<2, 4>(smem, &per_sm);
-  if (cblock == 8) return max_ctas<8, 4>(smem, &per_sm);
-  return max_ctas<4, 4>(smem, &per_sm);
+  const JoinKernel kern = variant(K, R, d, true, ctas_per_sm, cblock, &L);
+  return max_ctas(kern, ctas_per_sm, cblock, L.bytes, &per_sm);
 }
 
 cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int iter, int out_buf, float stop_rate,
@@ -848,36 +1168,17 @@ cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, 
                         const int32_t* ids_in, const int32_t* scores_in, int32_t* ids_out, int32_t* scores_out,
                         const int32_t* row_order, unsigned long long* counters, int num_sms, cudaStream_t s,
                         const JobTable* jt, const JoinCtl* ctl, int ctas_per_sm, int cblock, int sk_words) {
-  const size_t smem = join_smem(K, R, d).bytes;
-  const JobTable no_jobs{};
-  const JoinCtl no_ctl{};
-  cudaError_t e = cudaSuccess;
-  auto go = [&](auto kern, cudaError_t qe, int max_per_sm) {
-    if (qe != cudaSuccess) {
-      e = qe;
-      return;
-    }
-    const int64_t blocks = std::min<int64_t>(n, int64_t(num_sms) * max_per_sm);
-    cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-    kern<<<unsigned(blocks), kThreads, smem, s>>>(codes, sketch, n, d, K, R, sk_words > 0 ? sk_words : d / 64, ids_in,
-                                                  scores_in, ids_out, scores_out, row_order, counters,
-                                                  jt ? *jt : no_jobs, ctl ? *ctl : no_ctl);
-    e = cudaGetLastError();
-  };
-  // ctas_per_sm 3: up to 85 registers per thread (no spills), 3 resident CTAs;
-  // otherwise 64 registers, 4 resident CTAs
+  JoinLayout L;
+  const JoinKernel kern = variant(K, R, d, (reinterpret_cast<uintptr_t>(ids_in) & 7) == 0, ctas_per_sm, cblock, &L);
   int per_sm = 1;
-  if (ctas_per_sm == 3) {
-    if (cblock == 2) { cudaError_t q = max_ctas<2, 3>(smem, &per_sm); go(join_kernel<2, 3>, q, per_sm); }
-    else if (cblock == 8) { cudaError_t q = max_ctas<8, 3>(smem, &per_sm); go(join_kernel<8, 3>, q, per_sm); }
-    else { cudaError_t q = max_ctas<4, 3>(smem, &per_sm); go(join_kernel<4, 3>, q, per_sm); }
-  } else {
-    if (cblock == 2) { cudaError_t q = max_ctas<2, 4>(smem, &per_sm); go(join_kernel<2, 4>, q, per_sm); }
-    else if (cblock == 8) { cudaError_t q = max_ctas<8, 4>(smem, &per_sm); go(join_kernel<8, 4>, q, per_sm); }
-    else { cudaError_t q = max_ctas<4, 4>(smem, &per_sm); go(join_kernel<4, 4>, q, per_sm); }
-  }
+  KNNG_CUDA_TRY(max_ctas(kern, ctas_per_sm, cblock, L.bytes, &per_sm));
+  const int64_t blocks = std::min<int64_t>(n, int64_t(num_sms) * per_sm);
+  cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
+  kern<<<unsigned(blocks), kThreads, L.bytes, s>>>(codes, sketch, n, d, K, R, sk_words > 0 ? sk_words : d / 64, ids_in,
+                                                   scores_in, ids_out, scores_out, row_order, counters,
+                                                   jt ? *jt : JobTable{}, ctl ? *ctl : JoinCtl{}, L);
   note_launch();
-  return e;
+  return cudaGetLastError();
 }
 
 }  // namespace knng

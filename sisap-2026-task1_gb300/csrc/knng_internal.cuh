@@ -243,7 +243,7 @@ struct JoinCtl {
   // dot is known to be <= the row's pool threshold (which never falls), so the
   // next iteration gathers sketches and code rows only for new candidates.
   int32_t* cache_ids;             // [n][cache_cap]
-  uint16_t* cache_hr;             // [n][cache_cap]: score << 1 | rejected
+  uint16_t* cache_hr;             // [n][cache_cap]: Hamming distance | rejected << 12
   int* cache_cnt;                 // [n]: entries held (0 before the first iteration)
   int cache_cap;
   int64_t row_limit;              // rows processed (the first ones in visit order); 0: all
@@ -281,7 +281,6 @@ cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, 
 // does nothing.
 cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int iter, int out_buf,
                               float stop_rate, float diff_tol, cudaStream_t s);
-int join_max_ctas_per_sm(int K, int R, int d);
 // Resolve a join variant's launch attributes before any stream capture.
 cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock);
 cudaError_t join_prepare_all(int K, int R, int d);  // every variant the autotuner may pick
