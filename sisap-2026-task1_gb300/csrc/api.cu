@@ -437,13 +437,16 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
   const int K = p.k_build, T = p.num_trees, W = d / 64, MI = p.max_iterations;
   std::memset(&S, 0, sizeof(S));
   std::vector<int32_t> hoff(J), hn(J);
-  int64_t N = 0;
+  int64_t N = 0, root_tiles = 0;
   int split = 0;
   for (int b = 0; b < J; ++b) {
     hoff[b] = int32_t(N);
     hn[b] = int32_t(jobs[b].n);
     N += jobs[b].n;
-    if (jobs[b].n > p.leaf_size) ++split;
+    if (jobs[b].n > p.leaf_size) {
+      ++split;
+      root_tiles += forest_tiles(jobs[b].n);
+    }
   }
   if (int64_t(T) * N > INT32_MAX) return set_error(c, KNNG_E_ARGS, "num_trees * total rows must fit in int32");
   cudaError_t e;
@@ -533,7 +536,7 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
     }
   } else if ((st = run_forest(c->codes.as<int8_t>(), N, d, T, p.leaf_size, p.seed, nullptr, 0, c->perm.as<int32_t>(),
                               c->leaf_flag.as<uint8_t>(), s.fb, str, &levels, &c->last_error, jt, split,
-                              p.forest_fuse))) {
+                              root_tiles, p.forest_fuse))) {
     return st;
   }
   cudaEventRecord(c->ev[2], str);
@@ -864,7 +867,7 @@ int knng_forest(knng_ctx* c, const int8_t* codes_dev, int64_t n, int d, const in
     if ((st = single_job(c, n, &jt))) return st;
     st = run_forest(codes_dev, n, d, c->prm.num_trees, c->prm.leaf_size, c->prm.seed, replay, replay ? n_replay : 0,
                     perm_dev, leaf_flag_dev, s.fb, c->stream, &levels, &c->last_error, jt,
-                    n > c->prm.leaf_size ? 1 : 0, c->prm.forest_fuse);
+                    n > c->prm.leaf_size ? 1 : 0, n > c->prm.leaf_size ? forest_tiles(n) : 0, c->prm.forest_fuse);
     if (st) return st;
     cudaError_t e = cudaStreamSynchronize(c->stream);
     return e ? cuda_fail(c, e, "forest") : KNNG_OK;

@@ -45,8 +45,13 @@
 // is a contiguous range, left before right, as the per-level splits would
 // leave it (inside a descendant that turns out to be a leaf the members
 // are also ordered by the deeper bits, which no later stage depends on).
-// Nodes smaller than kFuseMin take the per-level path after the fused
-// rounds (the sample would be a large fraction of them).
+// Nodes smaller than kFuseMin are parked (the sample would be a large
+// fraction of them) and split to their leaves by one kernel after the fused
+// rounds, one CTA per node (subtree_kernel), with the per-level rule's pivots
+// and stable splits.
+//
+// Node lists are filled through atomic counters, so their order varies; a
+// node's pivots depend on its identity only, so the forest does not.
 #include "knng_internal.cuh"
 
 #include <algorithm>
@@ -69,6 +74,14 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   return x ^ (x >> 31);
 }
 
+// The hash a node's pivots are drawn from: its identity (tree, start within
+// the job's range, size) and the seed.
+__device__ __forceinline__ uint64_t node_hash(uint32_t seed, int32_t tree, int32_t local, int32_t size) {
+  uint64_t h = splitmix64((uint64_t(seed) << 32) ^ uint64_t(uint32_t(tree)));
+  h = splitmix64(h ^ uint64_t(uint32_t(local)));
+  return splitmix64(h ^ (uint64_t(uint32_t(size)) << 1));
+}
+
 struct NodeArr {
   int32_t *start, *size, *p1, *p2;
 };
@@ -84,14 +97,18 @@ __global__ void init_perm(int32_t* perm, int64_t n, int T) {
 
 // Roots: for tree t and job b the range t*N + off[b] of size n[b]; jobs with
 // n[b] <= leaf are single leaves.  Node order is by start (tree, then job).
-__global__ void root_nodes(NodeArr nd, int64_t N, int T, int leaf, uint8_t* leaf_flag, JobTable jt, int split_jobs) {
+// For the fused rounds p1 holds a root's first tile (root_tiles per tree).
+__global__ void root_nodes(NodeArr nd, int64_t N, int T, int leaf, uint8_t* leaf_flag, JobTable jt, int split_jobs,
+                           int root_tiles) {
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    int k = t * split_jobs;
+    int k = t * split_jobs, tile = t * root_tiles;
     for (int b = 0; b < jt.count; ++b) {
       const int64_t start = int64_t(t) * N + jt.off[b];
       if (jt.n[b] > leaf) {
         nd.start[k] = int32_t(start);
         nd.size[k] = jt.n[b];
+        nd.p1[k] = tile;
+        tile += (jt.n[b] + kTileElems - 1) / kTileElems;
         ++k;
       } else {
         leaf_flag[start] = 1;
@@ -122,9 +139,7 @@ __global__ void pick_pivots(NodeArr nd, int cnt, int64_t n, uint32_t seed, int l
       p2 = r[5];
     }
   } else {
-    uint64_t h = splitmix64((uint64_t(seed) << 32) ^ uint64_t(uint32_t(tree)));
-    h = splitmix64(h ^ uint64_t(uint32_t(local)));
-    h = splitmix64(h ^ (uint64_t(uint32_t(size)) << 1));
+    const uint64_t h = node_hash(seed, tree, local, size);
     const uint64_t h2 = splitmix64(h ^ 0x5851F42D4C957F2Dull);
     int32_t a = int32_t(h % uint64_t(size));
     int32_t b = int32_t(h2 % uint64_t(size - 1));
@@ -330,13 +345,20 @@ __global__ void chunk_leaves(NodeArr nd, int cnt, int leaf, uint8_t* leaf_flag) 
 
 // ---- fused levels ------------------------------------------------------------
 
-__device__ __forceinline__ int64_t gcd64(int64_t a, int64_t b) {
+__device__ __forceinline__ uint32_t gcd32(uint32_t a, uint32_t b) {
   while (b) {
-    const int64_t t = a % b;
+    const uint32_t t = a % b;
     a = b;
     b = t;
   }
   return a;
+}
+
+__device__ __forceinline__ int dot16(uint4 v, uint4 a, int acc) {
+  acc = __dp4a(int(v.x), int(a.x), acc);
+  acc = __dp4a(int(v.y), int(a.y), acc);
+  acc = __dp4a(int(v.z), int(a.z), acc);
+  return __dp4a(int(v.w), int(a.w), acc);
 }
 
 // 8-lane partial dot of a member row (v: chunks sub, sub+8, ... in registers)
@@ -356,99 +378,105 @@ __device__ __forceinline__ int dot_chunks(const uint4* v, const uint4* row, int 
   return acc;
 }
 
-// Pivot table of fused node k, one warp per node: piv[k][2j], piv[k][2j+1]
+// Pivot table of fused node k, one CTA per node: piv[k][2j], piv[k][2j+1]
 // are the pivots of descendant j (j = 0 the node; 2j+1 and 2j+2 the left and
 // right children of j), or -1 where j is not split in the pass.  The node's
 // candidates are the members at positions a + q*b (mod size), q < S, with b
 // coprime to size (distinct positions), in q order; node identity is
-// job-local, as for pick_pivots.
+// job-local, as for pick_pivots.  Warp 0 chooses the pivots; the candidates'
+// sides are split over the 32 8-lane groups (two steps per level: with one
+// warp per node the first rounds, a few nodes each, waited 100 us for 16
+// steps of dependent gathers).  The CTA also fills the node's part of the
+// tile -> node map.
 __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t n, uint32_t seed,
                                                    const int32_t* __restrict__ perm,
                                                    const int8_t* __restrict__ codes, int d,
-                                                   int32_t* __restrict__ piv, int32_t* __restrict__ tile_cnt,
-                                                   JobTable jt) {
-  __shared__ int32_t s_side[8][kCand];
-  __shared__ int32_t s_pv[8][2 * kFuseNodes];
+                                                   int32_t* __restrict__ piv, int32_t* __restrict__ tile_node,
+                                                   int64_t tile_cap, unsigned* err, JobTable jt) {
+  __shared__ int32_t s_id[kCand];
+  __shared__ int32_t s_node[kCand];
+  __shared__ int32_t s_side[kCand];
+  __shared__ int32_t s_pv[2 * kFuseNodes];
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & 7, slot = lane >> 3;
-  const int64_t k = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  if (k >= cnt) return;  // whole warps
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, sub = lane & 7, slot = lane >> 3;
+  const int k = blockIdx.x;
   const int32_t start = nd.start[k], size = nd.size[k];
-  const int32_t tree = int32_t(int64_t(start) / n);
-  const int32_t in_tree = int32_t(int64_t(start) - int64_t(tree) * n);
-  const int32_t local = in_tree - jt.off[job_of(jt, in_tree)];
-  uint64_t h = splitmix64((uint64_t(seed) << 32) ^ uint64_t(uint32_t(tree)));
-  h = splitmix64(h ^ uint64_t(uint32_t(local)));
-  h = splitmix64(h ^ (uint64_t(uint32_t(size)) << 1));
-  const uint64_t h2 = splitmix64(h ^ 0x2545F4914F6CDD1Dull);
-  const int64_t a = int64_t(h % uint64_t(size));
-  int64_t b = 1 + int64_t(h2 % uint64_t(size - 1));  // size > leaf_size >= 2
-  while (gcd64(b, size) != 1) b = b + 1 == size ? 1 : b + 1;
   const int S = size < kCand ? int(size) : kCand;
-  int32_t cid[2];
-  int cnode[2];
-  bool cused[2];
+  int32_t cid[2] = {-1, -1};
+  int cnode[2] = {-1, -1};
+  bool cused[2] = {false, false};
+  if (w == 0) {
+    const int32_t tree = int32_t(int64_t(start) / n);
+    const int32_t in_tree = int32_t(int64_t(start) - int64_t(tree) * n);
+    const uint64_t h = node_hash(seed, tree, in_tree - jt.off[job_of(jt, in_tree)], size);
+    const uint64_t h2 = splitmix64(h ^ 0x2545F4914F6CDD1Dull);
+    const int64_t a = int64_t(h % uint64_t(size));
+    int32_t b = 1 + int32_t(h2 % uint64_t(size - 1));  // size > leaf_size >= 2
+    while (gcd32(uint32_t(b), uint32_t(size)) != 1) b = b + 1 == size ? 1 : b + 1;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int q = lane + 32 * u;
-    cused[u] = false;
-    if (q < S) {
-      cid[u] = perm[start + (a + int64_t(q) * b) % size];
-      cnode[u] = 0;
+    for (int u = 0; u < 2; ++u) {
+      const int q = lane + 32 * u;
+      if (q < S) {
+        cid[u] = perm[start + (a + int64_t(q) * b) % size];
+        cnode[u] = 0;
+      }
+      s_id[q] = cid[u];
+      s_node[q] = cnode[u];
+    }
+    if (lane < 2 * kFuseNodes) s_pv[lane] = -1;
+  } else {
+    const int32_t f = nd.p1[k], nt = (size + kTileElems - 1) / kTileElems;
+    if (f + int64_t(nt) > tile_cap) {  // cannot happen: tiles are counted against max_tiles
+      if (tid == 32) atomicOr(err, kErrBounds);
     } else {
-      cid[u] = -1;
-      cnode[u] = -1;
+      for (int t = tid - 32; t < nt; t += 224) tile_node[f + t] = k;
     }
   }
-  if (lane < 2 * kFuseNodes) s_pv[w][lane] = -1;
-  __syncwarp();
   const int per_lane = d / 128;
   for (int dk = 0; dk < kFuse; ++dk) {
     const int j0 = (1 << dk) - 1;
-    // pivots of the depth-dk nodes: the two lowest-q free candidates in each
-    for (int j = j0; j < 2 * j0 + 1; ++j) {
-      const unsigned m0 = __ballot_sync(full, cnode[0] == j && !cused[0]);
-      const unsigned m1 = __ballot_sync(full, cnode[1] == j && !cused[1]);
-      uint64_t m = uint64_t(m0) | (uint64_t(m1) << 32);
-      if (__popcll(m) >= 2) {  // warp-uniform
-        const int q1 = __ffsll(m) - 1;
-        m &= m - 1;
-        const int q2 = __ffsll(m) - 1;
-        const int32_t p1 = __shfl_sync(full, (q1 >> 5) ? cid[1] : cid[0], q1 & 31);
-        const int32_t p2 = __shfl_sync(full, (q2 >> 5) ? cid[1] : cid[0], q2 & 31);
-        if (lane == (q1 & 31)) cused[q1 >> 5] = true;
-        if (lane == (q2 & 31)) cused[q2 >> 5] = true;
-        if (lane == 0) {
-          s_pv[w][2 * j] = p1;
-          s_pv[w][2 * j + 1] = p2;
+    if (w == 0) {
+      __syncwarp();
+      // pivots of the depth-dk nodes: the two lowest-q free candidates in each
+      for (int j = j0; j < 2 * j0 + 1; ++j) {
+        const unsigned m0 = __ballot_sync(full, cnode[0] == j && !cused[0]);
+        const unsigned m1 = __ballot_sync(full, cnode[1] == j && !cused[1]);
+        uint64_t m = uint64_t(m0) | (uint64_t(m1) << 32);
+        if (__popcll(m) >= 2) {  // warp-uniform
+          const int q1 = __ffsll(m) - 1;
+          m &= m - 1;
+          const int q2 = __ffsll(m) - 1;
+          const int32_t p1 = __shfl_sync(full, (q1 >> 5) ? cid[1] : cid[0], q1 & 31);
+          const int32_t p2 = __shfl_sync(full, (q2 >> 5) ? cid[1] : cid[0], q2 & 31);
+          if (lane == (q1 & 31)) cused[q1 >> 5] = true;
+          if (lane == (q2 & 31)) cused[q2 >> 5] = true;
+          if (lane == 0) {
+            s_pv[2 * j] = p1;
+            s_pv[2 * j + 1] = p2;
+          }
         }
       }
     }
-    __syncwarp();
+    __syncthreads();
     if (dk + 1 == kFuse) break;  // no pivots below the last fused level
     // every candidate in a split depth-dk node takes its side (8 lanes per candidate)
-    for (int g = 0; g < S; g += 4) {
-      const int q = g + slot, half = g >> 5;  // g % 4 == 0: the 4 candidates share a half
-      const int32_t myid = __shfl_sync(full, half ? cid[1] : cid[0], q & 31);
-      const int jn = __shfl_sync(full, half ? cnode[1] : cnode[0], q & 31);
-      const int32_t p1 = (q < S && jn >= 0) ? s_pv[w][2 * jn] : -1;
-      const int32_t p2 = (q < S && jn >= 0) ? s_pv[w][2 * jn + 1] : -1;
+    for (int g = 4 * w; g < S; g += 32) {  // warp-uniform trip count
+      const int q = g + slot;  // < kCand
+      const int32_t myid = s_id[q];
+      const int jn = s_node[q];
+      const int32_t p1 = jn >= 0 ? s_pv[2 * jn] : -1;
+      const int32_t p2 = jn >= 0 ? s_pv[2 * jn + 1] : -1;
       const bool live = p1 >= 0;
       int d1 = 0, d2 = 0;
       if (live) {
         const uint4* x = reinterpret_cast<const uint4*>(codes + int64_t(myid) * d);
         const uint4* r1 = reinterpret_cast<const uint4*>(codes + int64_t(p1) * d);
         const uint4* r2 = reinterpret_cast<const uint4*>(codes + int64_t(p2) * d);
+#pragma unroll 4
         for (int u = 0; u < per_lane; ++u) {
           const uint4 xv = __ldg(x + sub + 8 * u), av = __ldg(r1 + sub + 8 * u), cv = __ldg(r2 + sub + 8 * u);
-          d1 = __dp4a(int(xv.x), int(av.x), d1);
-          d1 = __dp4a(int(xv.y), int(av.y), d1);
-          d1 = __dp4a(int(xv.z), int(av.z), d1);
-          d1 = __dp4a(int(xv.w), int(av.w), d1);
-          d2 = __dp4a(int(xv.x), int(cv.x), d2);
-          d2 = __dp4a(int(xv.y), int(cv.y), d2);
-          d2 = __dp4a(int(xv.z), int(cv.z), d2);
-          d2 = __dp4a(int(xv.w), int(cv.w), d2);
+          d1 = dot16(xv, av, d1);
+          d2 = dot16(xv, cv, d2);
         }
       }
 #pragma unroll
@@ -457,21 +485,22 @@ __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t 
         d2 += __shfl_xor_sync(full, d2, o);
       }
       const int sd = myid == p1 ? 0 : myid == p2 ? 1 : (d1 > d2 ? 0 : 1);
-      if (sub == 0 && q < S) s_side[w][q] = live ? sd : -1;
+      if (sub == 0) s_side[q] = live ? sd : -1;
     }
-    __syncwarp();
+    __syncthreads();
+    if (w == 0) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int q = lane + 32 * u;
-      if (q < S && cnode[u] >= 0) {
-        const int sd = s_side[w][q];
-        cnode[u] = sd < 0 ? -1 : 2 * cnode[u] + 1 + sd;
+      for (int u = 0; u < 2; ++u) {
+        const int q = lane + 32 * u;
+        if (q < S && cnode[u] >= 0) {
+          const int sd = s_side[q];
+          cnode[u] = sd < 0 ? -1 : 2 * cnode[u] + 1 + sd;
+          s_node[q] = cnode[u];
+        }
       }
     }
-    __syncwarp();
   }
-  if (lane < 2 * kFuseNodes) piv[k * (2 * kFuseNodes) + lane] = s_pv[w][lane];
-  if (lane == 0) tile_cnt[k] = (size + kTileElems - 1) / kTileElems;
+  if (tid < 2 * kFuseNodes) piv[int64_t(k) * (2 * kFuseNodes) + tid] = s_pv[tid];
 }
 
 // Member pass of the fused levels: one block per tile of <= 256 members of one
@@ -481,20 +510,17 @@ __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t 
 // count, at bins[8*f + code*nt + (tile - f)] (f: the node's first tile, nt:
 // its tile count), so one exclusive scan of bins gives every member's place.
 __global__ void __launch_bounds__(256) fuse_side(const int8_t* __restrict__ codes, int d,
-                                                 const int32_t* __restrict__ perm, NodeArr nd, int cnt,
-                                                 const int32_t* __restrict__ tile_off,
+                                                 const int32_t* __restrict__ perm, NodeArr nd,
+                                                 const int32_t* __restrict__ tile_node,
                                                  const int32_t* __restrict__ piv, uint8_t* __restrict__ side,
                                                  int32_t* __restrict__ bins) {
   __shared__ uint4 prow[2 * kFuseNodes][kMaxDim / 16];
   __shared__ int32_t spv[2 * kFuseNodes];
   __shared__ int32_t sbins[kFuseBins];
-  __shared__ int node_s;
   const unsigned full = 0xffffffffu;
   const int b = blockIdx.x, tid = threadIdx.x;
-  if (tid == 0) node_s = find_node(tile_off, cnt, b);
+  const int k = tile_node[b];
   if (tid < kFuseBins) sbins[tid] = 0;
-  __syncthreads();
-  const int k = node_s;
   if (tid < 2 * kFuseNodes) spv[tid] = piv[int64_t(k) * (2 * kFuseNodes) + tid];
   __syncthreads();
   const int nchunk = d / 16;
@@ -505,7 +531,7 @@ __global__ void __launch_bounds__(256) fuse_side(const int8_t* __restrict__ code
   }
   __syncthreads();
   const int32_t start = nd.start[k], size = nd.size[k];
-  const int f = tile_off[k], nt = (size + kTileElems - 1) / kTileElems;
+  const int f = nd.p1[k], nt = (size + kTileElems - 1) / kTileElems;
   const int64_t e0 = int64_t(start) + int64_t(b - f) * kTileElems;
   const int64_t e1 = min(int64_t(start) + size, e0 + kTileElems);
   const int lane = tid & 31, warp = tid >> 5, sub = lane & 7, slot = lane >> 3;
@@ -557,18 +583,15 @@ __global__ void __launch_bounds__(256) fuse_side(const int8_t* __restrict__ code
 
 // Stable counting sort of each node's members by path code into perm_tmp.
 __global__ void __launch_bounds__(256) fuse_scatter(const int32_t* __restrict__ perm,
-                                                    int32_t* __restrict__ perm_tmp, NodeArr nd, int cnt,
-                                                    const int32_t* __restrict__ tile_off,
+                                                    int32_t* __restrict__ perm_tmp, NodeArr nd,
+                                                    const int32_t* __restrict__ tile_node,
                                                     const uint8_t* __restrict__ side,
                                                     const int32_t* __restrict__ bins_off) {
-  __shared__ int node_s;
   __shared__ int32_t wcnt[8][kFuseBins];
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) node_s = find_node(tile_off, cnt, b);
-  __syncthreads();
-  const int k = node_s;
+  const int k = tile_node[b];
   const int32_t start = nd.start[k], size = nd.size[k];
-  const int f = tile_off[k], nt = (size + kTileElems - 1) / kTileElems;
+  const int f = nd.p1[k], nt = (size + kTileElems - 1) / kTileElems;
   const int64_t e0 = int64_t(start) + int64_t(b - f) * kTileElems;
   const int64_t e1 = min(int64_t(start) + size, e0 + kTileElems);
   const int64_t e = e0 + tid;
@@ -591,20 +614,27 @@ __global__ void __launch_bounds__(256) fuse_scatter(const int32_t* __restrict__ 
   }
 }
 
+// perm takes the sorted members over.
+__global__ void __launch_bounds__(256) fuse_copyback(int32_t* __restrict__ perm, const int32_t* __restrict__ perm_tmp,
+                                                     NodeArr nd, const int32_t* __restrict__ tile_node) {
+  const int b = blockIdx.x, k = tile_node[b];
+  const int64_t start = nd.start[k];
+  const int64_t e = start + int64_t(b - nd.p1[k]) * kTileElems + threadIdx.x;
+  if (e < start + nd.size[k]) perm[e] = perm_tmp[e];
+}
+
 // After a fused pass: the sizes of node k's descendants from the scanned code
 // counts; leaves are flagged, and every descendant that is neither a leaf nor
 // split in the pass becomes a node: of the next fused round when it has at
-// least kFuseMin members, else of the per-level phase.  emit = 0 counts them
-// per node (and sets the leaf flags), emit = 1 writes them at the scanned
-// offsets.
-__global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __restrict__ tile_off,
-                              const int32_t* __restrict__ bins_off, const int32_t* __restrict__ piv,
-                              uint8_t* __restrict__ leaf_flag, int emit, int32_t* cnt_big, int32_t* cnt_small,
-                              NodeArr big, NodeArr small, int64_t small_base, int64_t cap, unsigned* err) {
+// least kFuseMin members (with its tiles reserved), else parked for the
+// subtree kernel.  counts: nodes of the next round, their tiles, parked nodes.
+__global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __restrict__ bins_off,
+                              const int32_t* __restrict__ piv, uint8_t* __restrict__ leaf_flag, int32_t* counts,
+                              NodeArr big, NodeArr small, int64_t cap, unsigned* err) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
   const int32_t start = nd.start[k], size = nd.size[k];
-  const int f = tile_off[k], nt = (size + kTileElems - 1) / kTileElems;
+  const int f = nd.p1[k], nt = (size + kTileElems - 1) / kTileElems;
   const int64_t base = int64_t(8) * f;
   int32_t pre[kFuseBins + 1];
   pre[0] = 0;
@@ -614,8 +644,6 @@ __global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __re
   bool split[kFuseNodes];
 #pragma unroll
   for (int j = 0; j < kFuseNodes; ++j) split[j] = j == 0;
-  int64_t ob = emit ? cnt_big[k] : 0, os = emit ? small_base + cnt_small[k] : 0;
-  int nb = 0, ns = 0;
 #pragma unroll
   for (int j = 0; j < kFuseNodes; ++j) {
     if (!split[j]) continue;
@@ -629,41 +657,213 @@ __global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __re
       if (csize <= 0) {  // cannot happen: a split sends its two pivots to different sides
         atomicOr(err, kErrBounds);
       } else if (csize <= leaf) {
-        if (!emit) leaf_flag[cstart] = 1;
+        leaf_flag[cstart] = 1;
       } else if (cd < kFuse && piv[int64_t(k) * (2 * kFuseNodes) + 2 * ch] >= 0) {
         split[ch] = true;
-      } else if (csize >= kFuseMin) {
-        if (emit) {
-          if (ob >= cap) {
-            atomicOr(err, kErrBounds);
-          } else {
-            big.start[ob] = int32_t(cstart);
-            big.size[ob] = csize;
-          }
-        }
-        ++ob;
-        ++nb;
       } else {
-        if (emit) {
-          if (os >= cap) {
-            atomicOr(err, kErrBounds);
-          } else {
-            small.start[os] = int32_t(cstart);
-            small.size[os] = csize;
-          }
+        const bool is_big = csize >= kFuseMin;
+        const int o = atomicAdd(counts + (is_big ? 0 : 2), 1);
+        if (o >= cap) {  // cannot happen: active nodes are disjoint and larger than leaf
+          atomicOr(err, kErrBounds);
+        } else if (is_big) {
+          big.start[o] = int32_t(cstart);
+          big.size[o] = csize;
+          big.p1[o] = atomicAdd(counts + 1, (csize + kTileElems - 1) / kTileElems);
+        } else {
+          small.start[o] = int32_t(cstart);
+          small.size[o] = csize;
         }
-        ++os;
-        ++ns;
       }
     }
   }
-  if (!emit) {
-    cnt_big[k] = nb;
-    cnt_small[k] = ns;
+}
+
+// Splits a parked node (fewer than kFuseMin members) down to its leaves, one
+// CTA per node, level by level over all of its open descendants: the per-level
+// rule's pivots (pick_pivots), stable splits and depth valve, with the node's
+// part of the permutation in shared memory.  8 lanes per member and level: the
+// member's row is read (by then from L2, for the most part), the pivot rows
+// are staged in shared memory while at most kSubStage descendants are open
+// (with the default leaf size at most 7 are).  It replaces 10 to 16 rounds of
+// 8 to 10 launches and two host waits each: with the wider fuse_pivots and one
+// wait per fused round the forest went from 0.97 to 0.24 ms at 2,000 x 384,
+// 4.71 to 2.66 ms at 100,000 x 1024 and 34.2 to 26.0 ms at 1M x 1024.
+constexpr int kSubStage = 16;
+constexpr int kSubNodes = 256;  // more open descendants than kFuseMin members can hold (each has at least 3)
+
+template <int PL>  // 16-byte chunks per lane: d / 128
+__global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__ codes, int32_t* __restrict__ perm,
+                                                      NodeArr nd, int64_t n, uint32_t seed, int leaf,
+                                                      uint8_t* __restrict__ leaf_flag, int level0,
+                                                      int32_t* __restrict__ max_level, JobTable jt) {
+  constexpr int d = 128 * PL;
+  extern __shared__ uint4 s_prow[];  // [2 * kSubStage][8 * PL]
+  __shared__ int32_t s_perm[2][kFuseMin];
+  __shared__ int16_t s_lpre[kFuseMin + 1];    // lefts before each position
+  __shared__ int16_t s_node[kFuseMin];        // open descendant of each position, -1: in a leaf
+  __shared__ uint8_t s_side[kFuseMin];
+  __shared__ int16_t s_start[2][kSubNodes], s_size[2][kSubNodes];
+  __shared__ int16_t s_nl[kSubNodes], s_cl[kSubNodes], s_cr[kSubNodes];
+  __shared__ int32_t s_p1[kSubNodes], s_p2[kSubNodes];
+  __shared__ int s_wcnt[16];
+  __shared__ int s_next;
+  __shared__ int32_t s_local;
+  const unsigned full = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7;
+  const int k0 = blockIdx.x;
+  const int32_t start = nd.start[k0], size = nd.size[k0];
+  const int32_t tree = int32_t(int64_t(start) / n);
+  if (tid == 0) {
+    const int32_t in_tree = int32_t(int64_t(start) - int64_t(tree) * n);
+    s_local = in_tree - jt.off[job_of(jt, in_tree)];
+    s_start[0][0] = 0;
+    s_size[0][0] = int16_t(size);
   }
+  for (int t = tid; t < size; t += 256) {
+    s_perm[0][t] = perm[int64_t(start) + t];
+    s_node[t] = 0;
+  }
+  int cnt = 1, cur = 0, level = level0;
+  __syncthreads();
+  while (cnt > 0) {  // a level closes every node it splits; children are smaller: ends
+    if (level >= kMaxLevels) {  // depth valve: the rest become consecutive leaves
+      for (int k = tid; k < cnt; k += 256)
+        for (int p = s_start[cur][k], e = p + s_size[cur][k]; p < e; p += leaf) leaf_flag[int64_t(start) + p] = 1;
+      break;
+    }
+    for (int k = tid; k < cnt; k += 256) {
+      const int32_t st = s_start[cur][k], sz = s_size[cur][k];
+      const uint64_t h = node_hash(seed, tree, s_local + st, sz);
+      const uint64_t h2 = splitmix64(h ^ 0x5851F42D4C957F2Dull);
+      const int32_t a = int32_t(h % uint64_t(sz));
+      int32_t b = int32_t(h2 % uint64_t(sz - 1));
+      if (b >= a) ++b;
+      s_p1[k] = s_perm[cur][st + a];
+      s_p2[k] = s_perm[cur][st + b];
+    }
+    __syncthreads();
+    if (tid == 0) s_next = 0;  // everyone has read it; counted up two barriers on
+    const bool staged = cnt <= kSubStage;
+    if (staged) {
+      for (int c = tid; c < 2 * cnt * 8 * PL; c += 256) {
+        const int r = c / (8 * PL), cc = c % (8 * PL);
+        const int32_t id = (r & 1) ? s_p2[r >> 1] : s_p1[r >> 1];
+        s_prow[c] = __ldg(reinterpret_cast<const uint4*>(codes + int64_t(id) * d) + cc);
+      }
+      __syncthreads();
+    }
+    for (int t0 = 0; t0 < size; t0 += 32) {  // 32 members per step, 4 per warp
+      const int t = t0 + (tid >> 3);
+      const int k = t < size ? int(s_node[t]) : -1;
+      if (!__any_sync(full, k >= 0)) continue;  // warp-uniform
+      int d1 = 0, d2 = 0;
+      int32_t id = -1;
+      if (k >= 0) {
+        id = s_perm[cur][t];
+        const uint4* row = reinterpret_cast<const uint4*>(codes + int64_t(id) * d) + sub;
+        uint4 v[PL];
+#pragma unroll
+        for (int u = 0; u < PL; ++u) v[u] = __ldg(row + 8 * u);
+        if (staged) {
+          const uint4* a = s_prow + (2 * k) * (8 * PL) + sub;
+#pragma unroll
+          for (int u = 0; u < PL; ++u) {
+            d1 = dot16(v[u], a[8 * u], d1);
+            d2 = dot16(v[u], a[8 * PL + 8 * u], d2);
+          }
+        } else {
+          const uint4* a = reinterpret_cast<const uint4*>(codes + int64_t(s_p1[k]) * d) + sub;
+          const uint4* c = reinterpret_cast<const uint4*>(codes + int64_t(s_p2[k]) * d) + sub;
+#pragma unroll
+          for (int u = 0; u < PL; ++u) {
+            d1 = dot16(v[u], __ldg(a + 8 * u), d1);
+            d2 = dot16(v[u], __ldg(c + 8 * u), d2);
+          }
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        d1 += __shfl_xor_sync(full, d1, o);
+        d2 += __shfl_xor_sync(full, d2, o);
+      }
+      if (sub == 0 && k >= 0) s_side[t] = (id == s_p1[k]) || (id != s_p2[k] && d1 > d2) ? 1 : 0;
+    }
+    __syncthreads();
+    // lefts before every position
+    unsigned bal[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = tid + 256 * u;
+      bal[u] = __ballot_sync(full, t < size && s_node[t] >= 0 && s_side[t]);
+      if (lane == 0) s_wcnt[8 * u + warp] = __popc(bal[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = tid + 256 * u;
+      int before = __popc(bal[u] & ((1u << lane) - 1u));
+      for (int w = 0; w < 8 * u + warp; ++w) before += s_wcnt[w];
+      if (t < size) s_lpre[t] = int16_t(before);
+      if (t == size - 1) s_lpre[size] = int16_t(before + int((bal[u] >> lane) & 1u));
+    }
+    __syncthreads();
+    for (int k = tid; k < cnt; k += 256) {
+      const int st = s_start[cur][k], sz = s_size[cur][k];
+      const int nl = s_lpre[st + sz] - s_lpre[st], nr = sz - nl;
+      s_nl[k] = int16_t(nl);
+      s_cl[k] = s_cr[k] = -1;
+      if (nl <= leaf) {
+        leaf_flag[int64_t(start) + st] = 1;
+      } else {
+        const int o = atomicAdd(&s_next, 1);
+        s_cl[k] = int16_t(o);
+        s_start[cur ^ 1][o] = int16_t(st);
+        s_size[cur ^ 1][o] = int16_t(nl);
+      }
+      if (nr <= leaf) {
+        leaf_flag[int64_t(start) + st + nl] = 1;
+      } else {
+        const int o = atomicAdd(&s_next, 1);
+        s_cr[k] = int16_t(o);
+        s_start[cur ^ 1][o] = int16_t(st + nl);
+        s_size[cur ^ 1][o] = int16_t(nr);
+      }
+    }
+    __syncthreads();
+    for (int t = tid; t < size; t += 256) {
+      const int k = s_node[t];
+      int np = t;
+      if (k >= 0) {
+        const int st = s_start[cur][k], l = s_lpre[t] - s_lpre[st];
+        np = s_side[t] ? st + l : st + s_nl[k] + (t - st - l);
+        s_node[t] = t - st < s_nl[k] ? s_cl[k] : s_cr[k];  // of position t, whoever moves there
+      }
+      s_perm[cur ^ 1][np] = s_perm[cur][t];
+    }
+    __syncthreads();
+    cnt = s_next;
+    cur ^= 1;
+    ++level;
+  }
+  for (int t = tid; t < size; t += 256) perm[int64_t(start) + t] = s_perm[cur][t];
+  if (tid == 0) atomicMax(max_level, level);
+}
+
+template <int PL>
+cudaError_t run_subtree(const int8_t* codes, int32_t* perm, const NodeArr& nd, int64_t cnt, int64_t n, uint32_t seed,
+                        int leaf, uint8_t* leaf_flag, int level0, int32_t* max_level, const JobTable& jt,
+                        cudaStream_t s) {
+  const size_t smem = size_t(2) * kSubStage * 128 * PL;
+  KNNG_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(subtree_kernel<PL>), smem));
+  cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
+  subtree_kernel<PL><<<unsigned(cnt), 256, smem, s>>>(codes, perm, nd, n, seed, leaf, leaf_flag, level0, max_level, jt);
+  note_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace
+
+int64_t forest_tiles(int64_t n) { return (n + kTileElems - 1) / kTileElems; }
 
 size_t forest_bytes(int64_t n, int T, int leaf, int64_t* max_nodes, int64_t* max_tiles) {
   const int64_t mn = int64_t(T) * (n / (leaf + 1) + 1) + 16;
@@ -683,7 +883,8 @@ size_t forest_bytes(int64_t n, int T, int leaf, int64_t* max_nodes, int64_t* max
 
 int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t seed, const int32_t* replay_host,
                int64_t n_replay, int32_t* perm, uint8_t* leaf_flag, const ForestBufs& fb, cudaStream_t s,
-               int64_t* levels_out, std::string* err, const JobTable& jt, int roots_with_split, int fuse) {
+               int64_t* levels_out, std::string* err, const JobTable& jt, int roots_with_split, int64_t root_tiles,
+               int fuse) {
   auto fail = [&](cudaError_t e, const char* what) {
     if (err) *err = std::string(what) + ": " + cudaGetErrorString(e);
     return int(KNNG_E_CUDA);
@@ -726,60 +927,52 @@ int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t 
   note_launch();
   NodeArr cur = node_arr(fb.node_a, fb.max_nodes), nxt = node_arr(fb.node_b, fb.max_nodes);
   cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-  root_nodes<<<1, 64, 0, s>>>(cur, n, T, leaf, leaf_flag, jt, roots_with_split);
+  root_nodes<<<1, 64, 0, s>>>(cur, n, T, leaf, leaf_flag, jt, roots_with_split, int(root_tiles));
   note_launch();
   int64_t cnt = int64_t(T) * roots_with_split;
   int level = 0;
   int64_t host_i64[3];
   if (fuse && !replay_host) {
     // fused rounds: kFuse levels per pass over nodes of >= kFuseMin members;
-    // smaller nodes collect in `parked` for the per-level loop below
+    // smaller nodes collect in `parked` for the subtree kernel.  The host only
+    // waits for the next round's node and tile counts.
     NodeArr parked = node_arr(fb.node_c, fb.max_nodes);
-    int64_t nparked = 0;
+    int32_t* counts = reinterpret_cast<int32_t*>(fb.dev_i64);  // next round's nodes, its tiles; parked nodes
+    int32_t* tile_node = fb.child_cnt2;  // at most one tile per leaf_size + 1 members: fits
+    int32_t host_cnt[3] = {0, 0, 0};
+    int64_t tiles = int64_t(T) * root_tiles;
+    if ((e = cudaMemsetAsync(fb.dev_i64, 0, 32, s))) return fail(e, "node counts");
     while (cnt > 0 && level < kMaxLevels) {
-      cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_pivots<<<grid1(cnt * 32), 256, 0, s>>>(cur, int(cnt), n, seed, perm, codes, d, fb.piv, fb.child_cnt,
-                                                   jt);
-      note_launch();
-      if ((e = exclusive_scan_i32(fb.child_cnt, fb.tile_off, cnt, fb.dev_i64, fb.scan_tmp, s))) return fail(e, "tile scan");
-      if ((e = cudaMemcpyAsync(host_i64, fb.dev_i64, 8, cudaMemcpyDeviceToHost, s))) return fail(e, "tile count");
-      if ((e = cudaStreamSynchronize(s))) return fail(e, "fused forest round");
-      const int64_t tiles = host_i64[0];
-      if (tiles > fb.max_tiles) {
+      if (tiles > fb.max_tiles || tiles > fb.max_nodes) {  // the tile -> node map has max_nodes entries
         if (err) *err = "forest tile overflow";
         return KNNG_E_ARGS;
       }
       cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_side<<<unsigned(tiles), 256, 0, s>>>(codes, d, perm, cur, int(cnt), fb.tile_off, fb.piv, fb.side,
-                                                fb.tile_bins);
+      fuse_pivots<<<unsigned(cnt), 256, 0, s>>>(cur, int(cnt), n, seed, perm, codes, d, fb.piv, tile_node,
+                                                fb.max_nodes, fb.err, jt);
+      note_launch();
+      cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
+      fuse_side<<<unsigned(tiles), 256, 0, s>>>(codes, d, perm, cur, tile_node, fb.piv, fb.side, fb.tile_bins);
       note_launch();
       if ((e = exclusive_scan_i32(fb.tile_bins, fb.tile_bins_off, int64_t(kFuseBins) * tiles, nullptr, fb.scan_tmp, s)))
         return fail(e, "code scan");
       cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_scatter<<<unsigned(tiles), 256, 0, s>>>(perm, fb.perm_tmp, cur, int(cnt), fb.tile_off, fb.side,
-                                                   fb.tile_bins_off);
+      fuse_children<<<grid1(cnt, 64), 64, 0, s>>>(cur, int(cnt), leaf, fb.tile_bins_off, fb.piv, leaf_flag, counts, nxt,
+                                                  parked, fb.max_nodes, fb.err);
       note_launch();
+      // the counts first: the next round is queued while the members are sorted
+      if ((e = cudaMemcpyAsync(host_cnt, counts, sizeof(host_cnt), cudaMemcpyDeviceToHost, s)) ||
+          (e = cudaStreamSynchronize(s)) || (e = cudaMemsetAsync(counts, 0, 2 * sizeof(int32_t), s)))
+        return fail(e, "fused forest round");
       cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      copyback_kernel<<<unsigned(tiles), 256, 0, s>>>(perm, fb.perm_tmp, cur, int(cnt), fb.tile_off);
+      fuse_scatter<<<unsigned(tiles), 256, 0, s>>>(perm, fb.perm_tmp, cur, tile_node, fb.side, fb.tile_bins_off);
       note_launch();
-      cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_children<<<grid1(cnt), 256, 0, s>>>(cur, int(cnt), leaf, fb.tile_off, fb.tile_bins_off, fb.piv, leaf_flag,
-                                               0, fb.child_cnt, fb.child_cnt2, nxt, parked, nparked, fb.max_nodes,
-                                               fb.err);
+      fuse_copyback<<<unsigned(tiles), 256, 0, s>>>(perm, fb.perm_tmp, cur, tile_node);
       note_launch();
-      if ((e = exclusive_scan_i32(fb.child_cnt, fb.child_cnt, cnt, fb.dev_i64 + 1, fb.scan_tmp, s)) ||
-          (e = exclusive_scan_i32(fb.child_cnt2, fb.child_cnt2, cnt, fb.dev_i64 + 2, fb.scan_tmp, s)))
-        return fail(e, "child scan");
-      cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_children<<<grid1(cnt), 256, 0, s>>>(cur, int(cnt), leaf, fb.tile_off, fb.tile_bins_off, fb.piv, leaf_flag,
-                                               1, fb.child_cnt, fb.child_cnt2, nxt, parked, nparked, fb.max_nodes,
-                                               fb.err);
-      note_launch();
-      if ((e = cudaMemcpyAsync(host_i64 + 1, fb.dev_i64 + 1, 16, cudaMemcpyDeviceToHost, s))) return fail(e, "child count");
-      if ((e = cudaStreamSynchronize(s))) return fail(e, "fused forest round");
-      cnt = host_i64[1];
-      nparked += host_i64[2];
-      if (cnt > fb.max_nodes || nparked > fb.max_nodes) {
+      if ((e = cudaGetLastError())) return fail(e, "fused forest round");
+      cnt = host_cnt[0];
+      tiles = host_cnt[1];
+      if (cnt > fb.max_nodes || host_cnt[2] > fb.max_nodes) {
         if (err) *err = "forest node overflow";
         return KNNG_E_ARGS;
       }
@@ -791,10 +984,25 @@ int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t 
       chunk_leaves<<<grid1(cnt), 256, 0, s>>>(cur, int(cnt), leaf, leaf_flag);
       note_launch();
     }
-    // the per-level loop takes the parked nodes
-    cnt = nparked;
-    nxt = cur.start == fb.node_a ? node_arr(fb.node_b, fb.max_nodes) : node_arr(fb.node_a, fb.max_nodes);
-    cur = parked;
+    cnt = 0;
+    if (host_cnt[2] > 0) {
+      int32_t* max_level = reinterpret_cast<int32_t*>(fb.dev_i64 + 3);
+      const int64_t parked_cnt = host_cnt[2];
+#define KNNG_SUBTREE(PL) \
+  case PL: e = run_subtree<PL>(codes, perm, parked, parked_cnt, n, seed, leaf, leaf_flag, level, max_level, jt, s); break;
+      switch (d / 128) {
+        KNNG_SUBTREE(1) KNNG_SUBTREE(2) KNNG_SUBTREE(3) KNNG_SUBTREE(4)
+        KNNG_SUBTREE(5) KNNG_SUBTREE(6) KNNG_SUBTREE(7) KNNG_SUBTREE(8)
+        default: e = cudaErrorInvalidValue;
+      }
+#undef KNNG_SUBTREE
+      if (e) return fail(e, "forest subtrees");
+      int32_t deepest = 0;
+      if ((e = cudaMemcpyAsync(&deepest, max_level, sizeof(int32_t), cudaMemcpyDeviceToHost, s)) ||
+          (e = cudaStreamSynchronize(s)))
+        return fail(e, "forest subtrees");
+      level = std::max(level, deepest);
+    }
   }
   while (cnt > 0) {
     if (level >= kMaxLevels) {
