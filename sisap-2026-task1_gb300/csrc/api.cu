@@ -53,8 +53,6 @@ void note_launch(int k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 
 using namespace knng;
 
-constexpr int kMaxIterEvents = 2 * 64 + 2;
-
 // A context-owned device buffer, allocated and freed in the order of the
 // context's stream (the device's stream-ordered pool), so growing or trimming
 // one context never synchronises the device under other contexts' work.
@@ -107,7 +105,6 @@ struct knng_ctx {
     if (pool) pool->copy(dst, src, bytes);
     else std::memcpy(dst, src, bytes);
   }
-  cudaEvent_t itev[kMaxIterEvents] = {};
   std::string last_error;
   DevBuf codes, sketch, graph, perm, leaf_flag, scratch, outbuf, scalars, jobs, hsketch, rowflags;
   // join phase captured as a CUDA graph, reused while the launch key matches
@@ -393,39 +390,94 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   return best;
 }
 
-// The NN-Descent phase: max_iterations launches of the join, each followed by
-// the per-job stop check; launches after every job has stopped do nothing.
-cudaError_t join_phase(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int32_t* const scs[2],
-                       const int32_t* order, const JobTable& jt, const JoinCtl& ctl, unsigned long long* counters,
-                       const JoinCfg& cfg, bool capture, const char** step) {
+// What the NN-Descent phase's launches share.
+struct JoinPhase {
+  int64_t N;
+  int d;
+  int32_t* ids[2];
+  int32_t* scs[2];
+  const int32_t* order;
+  JobTable jt;
+  JoinCtl ctl;
+  JoinCfg cfg;
+};
+
+// Launches iterations [from, to): a join and the per-job stop check each.
+// Iteration `it` reads buffer it % 2 (double-buffered mode); the device keeps
+// the iteration's number itself (JoinCtl::iter), so a loop may repeat a pair.
+cudaError_t join_iterations(knng_ctx* c, const JoinPhase& ph, int from, int to,
+                            const cudaGraphConditionalHandle* loop, const char** step) {
   const knng_params& p = c->prm;
   const int K = p.k_build;
   const bool jac = p.join_mode == KNNG_JOIN_JACOBI;
-  cudaError_t e;
-  int cur = 0;
-  for (int it = 0; it < p.max_iterations; ++it) {
-    const int nxt = jac ? 1 - cur : cur;
-    JoinCtl ci = ctl;  // this iteration's row-change flags: read the previous iteration's, write its own
+  for (int it = from; it < to; ++it) {
+    const int cur = jac ? it & 1 : 0, nxt = jac ? 1 - cur : 0;
+    JoinCtl ci = ph.ctl;  // this iteration's row-change flags: read the previous iteration's, write its own
     if (jac && c->rowflags.p) {
-      ci.chg_in = c->rowflags.as<uint8_t>(size_t(it & 1) * size_t(N));
-      ci.chg_out = c->rowflags.as<uint8_t>(size_t((it + 1) & 1) * size_t(N));
+      ci.chg_in = c->rowflags.as<uint8_t>(size_t(cur) * size_t(ph.N));
+      ci.chg_out = c->rowflags.as<uint8_t>(size_t(nxt) * size_t(ph.N));
     }
-    e = capture ? cudaEventRecordWithFlags(c->itev[2 * it], c->stream, cudaEventRecordExternal)
-                : cudaEventRecord(c->itev[2 * it], c->stream);
-    if (e) return (*step = "iteration start event", e);
-    if ((e = launch_join(c->codes.as<int8_t>(), c->join_sketch(), N, d, K, K * p.rerank_mult, ids[cur],
-                         scs[cur], ids[nxt], scs[nxt], order, counters + 8 * it, c->num_sms, c->stream, &jt, &ci,
-                         (it < 2 ? cfg.early : cfg.late).first, (it < 2 ? cfg.early : cfg.late).second,
-                         c->sketch_words(d))))
+    const auto& cfg = it < 2 ? ph.cfg.early : ph.cfg.late;
+    cudaError_t e;
+    if ((e = launch_join(c->codes.as<int8_t>(), c->join_sketch(), ph.N, ph.d, K, K * p.rerank_mult, ph.ids[cur],
+                         ph.scs[cur], ph.ids[nxt], ph.scs[nxt], ph.order, ph.ctl.counters, c->num_sms, c->stream,
+                         &ph.jt, &ci, cfg.first, cfg.second, c->sketch_words(ph.d))))
       return (*step = "join launch", e);
-    e = capture ? cudaEventRecordWithFlags(c->itev[2 * it + 1], c->stream, cudaEventRecordExternal)
-                : cudaEventRecord(c->itev[2 * it + 1], c->stream);
-    if (e) return (*step = "iteration end event", e);
-    if ((e = launch_stop_check(jt, ctl, K, it, nxt, p.early_stop_rate, p.rate_diff_tol, c->stream)))
+    if ((e = launch_stop_check(ph.jt, ph.ctl, K, nxt, p.early_stop_rate, p.rate_diff_tol, loop, c->stream)))
       return (*step = "stop check", e);
-    cur = nxt;
   }
   return cudaSuccess;
+}
+
+// The NN-Descent phase as a graph: iterations 0 and 1, then a loop node whose
+// body is iterations 2 and 3, repeated until the stop check says that every job
+// has stopped or max_iterations are done.  (A straight graph of 30 iterations
+// spent 0.33 ms on the launches after the last working one: as much as all of
+// the work at 2,000 rows.)  Null on failure; the caller then launches the
+// iterations one by one.
+cudaGraphExec_t capture_join_phase(knng_ctx* c, const JoinPhase& ph) {
+  const int MI = c->prm.max_iterations;
+  const cudaStream_t str = c->stream;
+  const char* step = "";
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  std::lock_guard<std::mutex> capture_lock(g_capture_mu);  // one capture at a time per process
+  if (cudaGraphCreate(&g, 0) != cudaSuccess) return nullptr;
+  auto captured = [&](cudaGraph_t to, int from, int upto, const cudaGraphConditionalHandle* loop,
+                      std::vector<cudaGraphNode_t>* last) {
+    if (cudaStreamBeginCaptureToGraph(str, to, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+      return false;
+    bool ok = join_iterations(c, ph, from, upto, loop, &step) == cudaSuccess;
+    if (last) {  // the nodes that the loop comes after
+      cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+      const cudaGraphNode_t* deps = nullptr;
+      size_t n = 0;
+      ok = ok && cudaStreamGetCaptureInfo(str, &status, nullptr, nullptr, &deps, nullptr, &n) == cudaSuccess &&
+           status == cudaStreamCaptureStatusActive;
+      if (ok) last->assign(deps, deps + n);
+    }
+    cudaGraph_t out = nullptr;
+    return cudaStreamEndCapture(str, &out) == cudaSuccess && ok;
+  };
+  cudaGraphConditionalHandle loop{};
+  std::vector<cudaGraphNode_t> last;
+  bool ok = true;
+  if (MI > 2) ok = cudaGraphConditionalHandleCreate(&loop, g, 0, cudaGraphCondAssignDefault) == cudaSuccess;
+  ok = ok && captured(g, 0, std::min(MI, 2), MI > 2 ? &loop : nullptr, MI > 2 ? &last : nullptr);
+  if (ok && MI > 2) {
+    cudaGraphNodeParams np{};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = loop;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    ok = cudaGraphAddNode(&node, g, last.data(), nullptr, last.size(), &np) == cudaSuccess &&
+         captured(np.conditional.phGraph_out[0], 2, 4, &loop, nullptr);
+  }
+  if (!ok || cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) exec = nullptr;
+  cudaGraphDestroy(g);
+  cudaGetLastError();
+  return exec;
 }
 
 // One problem made of J jobs of the same dimension d (a single build is J = 1).
@@ -466,14 +518,17 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
     o += (bytes + 15) & ~size_t(15);
     return at;
   };
+  // uploaded: off, n; read back in one copy: from the iteration counts on
   const size_t o_off = take(jb * 4), o_n = take(jb * 4), o_upd = take(jb * 8), o_done = take(jb * 4),
                o_prev = take(jb * 4), o_iters = take(jb * 4), o_flags = take(16), o_log = take(size_t(MI + 1) * jb * 8),
-               o_cnt = take(size_t(MI + 1) * 8 * 8);
+               o_times = take(size_t(MI + 1) * 16), o_cnt = take(size_t(MI + 1) * 8 * 8);
   if ((e = c->jobs.ensure(o))) return cuda_fail(c, e, "job table allocation");
   cudaStream_t str = c->stream;
-  if ((e = cudaMemsetAsync(c->jobs.p, 0, o, str)) ||
-      (e = cudaMemcpyAsync(c->jobs.as<int32_t>(o_off), hoff.data(), jb * 4, cudaMemcpyHostToDevice, str)) ||
-      (e = cudaMemcpyAsync(c->jobs.as<int32_t>(o_n), hn.data(), jb * 4, cudaMemcpyHostToDevice, str)))
+  std::vector<char> block(o);
+  std::memcpy(block.data() + o_off, hoff.data(), jb * 4);
+  std::memcpy(block.data() + o_n, hn.data(), jb * 4);
+  if ((e = cudaMemcpyAsync(c->jobs.p, block.data(), o_upd, cudaMemcpyHostToDevice, str)) ||
+      (e = cudaMemsetAsync(c->jobs.as<char>(o_upd), 0, o - o_upd, str)))
     return cuda_fail(c, e, "job table upload");
   JobTable jt;
   jt.count = J;
@@ -488,6 +543,9 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
   ctl.all_done = c->jobs.as<int>(o_flags);
   ctl.final_buf = c->jobs.as<int>(o_flags) + 1;
   ctl.upd_log = c->jobs.as<long long>(o_log);
+  ctl.iter = c->jobs.as<int>(o_flags) + 2;
+  ctl.max_iter = MI;
+  ctl.times = c->jobs.as<unsigned long long>(o_times);
   ctl.cache_ids = nullptr;
   ctl.cache_hr = nullptr;
   ctl.cache_cnt = nullptr;
@@ -572,6 +630,7 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
       (e = join_prepare(K, K * p.rerank_mult, d, cfg.late.first, cfg.late.second)))
     return cuda_fail(c, e, (std::string("join variant: ") + join_variant_error()).c_str());
   const char* step = "";
+  const JoinPhase ph{N, d, {ids[0], ids[1]}, {scs[0], scs[1]}, order, jt, ctl, cfg};
   if (p.use_graph) {
     const std::vector<uintptr_t> key = {uintptr_t(c->codes.p), uintptr_t(c->join_sketch()), uintptr_t(c->graph.p),
                                         uintptr_t(c->jobs.p), uintptr_t(c->perm.p), uintptr_t(ctl.cache_ids),
@@ -586,39 +645,26 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
         cudaGraphExecDestroy(c->join_graph);
         c->join_graph = nullptr;
       }
-      cudaGraph_t g = nullptr;
-      std::lock_guard<std::mutex> capture_lock(g_capture_mu);  // one capture at a time per process
-      if (cudaStreamBeginCapture(str, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const cudaError_t ce = join_phase(c, N, d, ids, scs, order, jt, ctl, ctl.counters, cfg, true, &step);
-        const cudaError_t ee = cudaStreamEndCapture(str, &g);
-        if (ce == cudaSuccess && ee == cudaSuccess && g &&
-            cudaGraphInstantiate(&c->join_graph, g, 0) == cudaSuccess)
-          c->join_graph_key = key;
-        else
-          c->join_graph = nullptr;
-        if (g) cudaGraphDestroy(g);
-      }
-      cudaGetLastError();
+      c->join_graph = capture_join_phase(c, ph);
+      if (c->join_graph) c->join_graph_key = key;
     }
     if (c->join_graph) {
       if ((e = cudaGraphLaunch(c->join_graph, str))) return cuda_fail(c, e, "join graph launch");
       graph_used = true;
     }
   }
-  if (!graph_used && (e = join_phase(c, N, d, ids, scs, order, jt, ctl, ctl.counters, cfg, false, &step)))
+  if (!graph_used && (e = join_iterations(c, ph, 0, MI, nullptr, &step)))
     return cuda_fail(c, e, (std::string("join phase (") + step + ")").c_str());
   cudaEventRecord(c->ev[4], str);
   // results of the control block
-  std::vector<int> iters(jb);
-  std::vector<long long> log(size_t(MI) * jb);
-  std::vector<unsigned long long> cnt(size_t(MI) * 8);
-  int flags[2] = {0, 0};
-  if ((e = cudaMemcpyAsync(iters.data(), ctl.job_iters, jb * 4, cudaMemcpyDeviceToHost, str)) ||
-      (MI && (e = cudaMemcpyAsync(log.data(), ctl.upd_log, log.size() * 8, cudaMemcpyDeviceToHost, str))) ||
-      (MI && (e = cudaMemcpyAsync(cnt.data(), ctl.counters, cnt.size() * 8, cudaMemcpyDeviceToHost, str))) ||
-      (e = cudaMemcpyAsync(flags, ctl.all_done, 8, cudaMemcpyDeviceToHost, str)) ||
+  if ((e = cudaMemcpyAsync(block.data() + o_iters, c->jobs.as<char>(o_iters), o - o_iters, cudaMemcpyDeviceToHost, str)) ||
       (e = cudaStreamSynchronize(str)))
     return cuda_fail(c, e, "join phase");
+  const int* iters = reinterpret_cast<const int*>(block.data() + o_iters);
+  const int* flags = reinterpret_cast<const int*>(block.data() + o_flags);
+  const long long* log = reinterpret_cast<const long long*>(block.data() + o_log);
+  const unsigned long long* times = reinterpret_cast<const unsigned long long*>(block.data() + o_times);
+  const unsigned long long* cnt = reinterpret_cast<const unsigned long long*>(block.data() + o_cnt);
   const int fin = MI == 0 ? 0 : flags[1];
   // export (job-local 1-based ids) and hand out each job's rows
   const size_t outn = size_t(N) * p.k_eval;
@@ -683,7 +729,7 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
     long long u = 0;
     for (int b = 0; b < J; ++b) u += log[size_t(it) * J + b];
     S.updates[it] = u;
-    S.join_ms[it] = elapsed(c->itev[2 * it], c->itev[2 * it + 1]);
+    S.join_ms[it] = double(times[2 * it + 1] - times[2 * it]) * 1e-6;
     S.join_candidates[it] = int64_t(cnt[8 * it + 1]);
     S.join_dots[it] = int64_t(cnt[8 * it + 2]);
     S.join_distinct[it] = int64_t(cnt[8 * it + 3]);
@@ -783,11 +829,6 @@ int knng_create(knng_ctx** out, const knng_params* p) {
         knng_destroy(c);
         return KNNG_E_CUDA;
       }
-    for (auto& ev : c->itev)
-      if ((e = cudaEventCreate(&ev))) {
-        knng_destroy(c);
-        return KNNG_E_CUDA;
-      }
     if ((e = cudaEventCreate(&c->bev))) {
       knng_destroy(c);
       return KNNG_E_CUDA;
@@ -817,8 +858,6 @@ void knng_destroy(knng_ctx* c) {
   if (c->join_graph) cudaGraphExecDestroy(c->join_graph);
   for (DevBuf* b : c->buffers()) b->release();
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (auto& ev : c->itev)
-    if (ev) cudaEventDestroy(ev);
   if (c->bev) cudaEventDestroy(c->bev);
   for (int k = 0; k < 2; ++k)
     if (c->freed[k]) cudaEventDestroy(c->freed[k]);

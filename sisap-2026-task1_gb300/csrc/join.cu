@@ -288,6 +288,12 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
   return v;
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 // CB: sketches in flight per 8-lane group (Hamming stage); MINB: resident CTAs
 // per SM the register budget allows; DEF: the default K and R (and 8-byte
 // aligned input lists), else any.
@@ -299,6 +305,12 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     const JoinLayout LA) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (ctl.all_done && *reinterpret_cast<volatile int*>(ctl.all_done)) return;
+  if (ctl.iter) {
+    const int it = *ctl.iter;
+    if (it >= ctl.max_iter) return;
+    counters += 8 * it;
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl.times[2 * it] = global_ns();
+  }
   constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim);
 #define KNNG_L(f) (DEF ? LD.f : LA.f)
   constexpr int NP = DEF ? (LD.pairs + kThreads - 1) / kThreads : kMaxPairs;  // pairs per thread
@@ -1052,27 +1064,35 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
 // rate < stop or (iter > 0 and prev - rate < diff).  When every job has
 // stopped, all_done is set and final_buf records the buffer that holds the
 // final graphs; later iterations of the launch sequence then do nothing.
-__global__ void stop_check_kernel(JobTable jt, JoinCtl ctl, int K, int iter, int out_buf, float stop_rate,
-                                  float diff_tol) {
-  if (*ctl.all_done) return;
+__global__ void stop_check_kernel(JobTable jt, JoinCtl ctl, int K, int out_buf, float stop_rate, float diff_tol,
+                                  cudaGraphConditionalHandle loop, int has_loop) {
+  const int iter = *ctl.iter;
   int all = 1;
-  for (int b = threadIdx.x; b < jt.count; b += blockDim.x) {
-    if (!ctl.job_done[b]) {
-      const unsigned long long upd = ctl.job_upd[b];
-      ctl.upd_log[int64_t(iter) * jt.count + b] = (long long)upd;
-      const float rate = float(upd) / float((unsigned long long)jt.n[b] * (unsigned long long)K);
-      const bool stop = rate < stop_rate || (iter > 0 && (ctl.job_prev[b] - rate) < diff_tol);
-      ctl.job_prev[b] = rate;
-      ctl.job_iters[b] = iter + 1;
-      ctl.job_upd[b] = 0;
-      if (stop) ctl.job_done[b] = 1;
-      else all = 0;
+  const bool ran = !*ctl.all_done && iter < ctl.max_iter;  // block-uniform: written below, behind a barrier
+  if (ran) {
+    if (threadIdx.x == 0) ctl.times[2 * iter + 1] = global_ns();
+    for (int b = threadIdx.x; b < jt.count; b += blockDim.x) {
+      if (!ctl.job_done[b]) {
+        const unsigned long long upd = ctl.job_upd[b];
+        ctl.upd_log[int64_t(iter) * jt.count + b] = (long long)upd;
+        const float rate = float(upd) / float((unsigned long long)jt.n[b] * (unsigned long long)K);
+        const bool stop = rate < stop_rate || (iter > 0 && (ctl.job_prev[b] - rate) < diff_tol);
+        ctl.job_prev[b] = rate;
+        ctl.job_iters[b] = iter + 1;
+        ctl.job_upd[b] = 0;
+        if (stop) ctl.job_done[b] = 1;
+        else all = 0;
+      }
     }
   }
   all = __syncthreads_and(all);
   if (threadIdx.x == 0) {
-    *ctl.final_buf = out_buf;
-    if (all) *ctl.all_done = 1;
+    if (ran) {
+      *ctl.iter = iter + 1;
+      *ctl.final_buf = out_buf;
+      if (all) *ctl.all_done = 1;
+    }
+    if (has_loop) cudaGraphSetConditional(loop, !all && iter + 1 < ctl.max_iter ? 1u : 0u);
   }
 }
 
@@ -1156,10 +1176,11 @@ cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock) {
   return max_ctas(kern, ctas_per_sm, cblock, L.bytes, &per_sm);
 }
 
-cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int iter, int out_buf, float stop_rate,
-                              float diff_tol, cudaStream_t s) {
+cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int out_buf, float stop_rate,
+                              float diff_tol, const cudaGraphConditionalHandle* loop, cudaStream_t s) {
   cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-  stop_check_kernel<<<1, 256, 0, s>>>(jt, ctl, K, iter, out_buf, stop_rate, diff_tol);
+  stop_check_kernel<<<1, 256, 0, s>>>(jt, ctl, K, out_buf, stop_rate, diff_tol, loop ? *loop : cudaGraphConditionalHandle{},
+                                      loop ? 1 : 0);
   note_launch();
   return cudaGetLastError();
 }

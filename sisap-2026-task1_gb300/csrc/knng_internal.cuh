@@ -255,6 +255,12 @@ struct JoinCtl {
   // before the first); the launch writes this iteration's flags to chg_out.
   const uint8_t* chg_in;
   uint8_t* chg_out;
+  // NN-Descent phase of a build (iter null: a single launch).  A launch works on
+  // iteration *iter (stop_check advances it), does nothing from max_iter on,
+  // and adds its counts to counters + 8 * iteration.
+  int* iter;
+  int max_iter;
+  unsigned long long* times;      // [max_iter][2]: start and end of each iteration's join, ns
   // error word of the bounds-checked build (null: none): an id outside [0, n)
   // in the input lists or the row order sets kErrBounds
   unsigned* check_err;
@@ -282,8 +288,10 @@ cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, 
 // With jt/ctl: rows of stopped jobs are copied through (when out != in) and
 // per-job updates are added to ctl->job_upd; if ctl->all_done is set the launch
 // does nothing.
-cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int iter, int out_buf,
-                              float stop_rate, float diff_tol, cudaStream_t s);
+// Per-job early stop after an iteration whose output is buffer out_buf; with a
+// conditional handle (null: none) it also decides whether the graph's loop goes on.
+cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int out_buf, float stop_rate,
+                              float diff_tol, const cudaGraphConditionalHandle* loop, cudaStream_t s);
 // Resolve a join variant's launch attributes before any stream capture.
 cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock);
 cudaError_t join_prepare_all(int K, int R, int d);  // every variant the autotuner may pick
