@@ -211,7 +211,8 @@ int run_init(const int8_t* codes, int64_t n, int d, int T, int leaf, int K, uint
              const int32_t* perm, const uint8_t* leaf_flag, int32_t* ids, int32_t* scores,
              const InitBufs& ib, cudaStream_t s, int64_t* leaves_out, std::string* err,
              const JobTable& jt, int gram_mode = 0, int wait_limit = 0);
-// gram_mode 0: dp4a leaf Gram (leaf_gram); 1: tcgen05 f16 tensor-core Gram (leaf_gram_tc)
+// gram_mode 0: dp4a leaf Gram (leaf_gram); 1: f16 tensor-core Gram (leaf_gram_mma, or with a
+// wait_limit the tcgen05 form leaf_gram_tc)
 // wait_limit: knng_params::wait_limit (0 = default polls per bounded wait)
 // Gram rows of the leaves [leaf_start, leaf_start + nleaves) (the last one ends
 // at position `total`) go to gram[(position - gram_pos0) * 64 ...].
@@ -219,6 +220,10 @@ cudaError_t launch_leaf_gram_tc(const int8_t* codes, int d, const int32_t* perm,
                                 int64_t nleaves, int64_t total, int32_t* gram, int64_t gram_pos0, unsigned* err,
                                 int num_sms, cudaStream_t s, int wait_limit, int64_t n_rows);
 // n_rows: rows of `codes` (the bounds-checked build checks every gathered id against it)
+// The same Gram rows by warp-level tensor-core instructions from registers (gram_mma.cu).
+cudaError_t launch_leaf_gram_mma(const int8_t* codes, int d, const int32_t* perm, const int32_t* leaf_start,
+                                 int64_t nleaves, int64_t total, int32_t* gram, int64_t gram_pos0, unsigned* err,
+                                 int num_sms, cudaStream_t s, int64_t n_rows);
 
 // Random initial graph (init_mode KNNG_INIT_RANDOM); every job needs n > K.
 cudaError_t launch_init_random(const int8_t* codes, int d, int64_t n_total, int K, uint32_t seed, const JobTable& jt,
