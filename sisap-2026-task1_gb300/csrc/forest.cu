@@ -361,23 +361,6 @@ __device__ __forceinline__ int dot16(uint4 v, uint4 a, int acc) {
   return __dp4a(int(v.w), int(a.w), acc);
 }
 
-// 8-lane partial dot of a member row (v: chunks sub, sub+8, ... in registers)
-// with a row in shared memory.
-__device__ __forceinline__ int dot_chunks(const uint4* v, const uint4* row, int sub, int per_lane) {
-  int acc = 0;
-#pragma unroll
-  for (int u = 0; u < kMaxDim / 128; ++u) {
-    if (u < per_lane) {
-      const uint4 a = row[sub + 8 * u];
-      acc = __dp4a(int(v[u].x), int(a.x), acc);
-      acc = __dp4a(int(v[u].y), int(a.y), acc);
-      acc = __dp4a(int(v[u].z), int(a.z), acc);
-      acc = __dp4a(int(v[u].w), int(a.w), acc);
-    }
-  }
-  return acc;
-}
-
 // Pivot table of fused node k, one CTA per node: piv[k][2j], piv[k][2j+1]
 // are the pivots of descendant j (j = 0 the node; 2j+1 and 2j+2 the left and
 // right children of j), or -1 where j is not split in the pass.  The node's
@@ -504,76 +487,148 @@ __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t 
 }
 
 // Member pass of the fused levels: one block per tile of <= 256 members of one
-// node, the node's (up to 14) pivot rows staged in shared memory; 8 lanes per
-// member hold its code row in registers and walk its path down the fused
-// levels.  side[e] = the member's path code; per tile and code the member
-// count, at bins[8*f + code*nt + (tile - f)] (f: the node's first tile, nt:
-// its tile count), so one exclusive scan of bins gives every member's place.
-__global__ void __launch_bounds__(256) fuse_side(const int8_t* __restrict__ codes, int d,
-                                                 const int32_t* __restrict__ perm, NodeArr nd,
-                                                 const int32_t* __restrict__ tile_node,
-                                                 const int32_t* __restrict__ piv, uint8_t* __restrict__ side,
-                                                 int32_t* __restrict__ bins) {
-  __shared__ uint4 prow[2 * kFuseNodes][kMaxDim / 16];
-  __shared__ int32_t spv[2 * kFuseNodes];
+// node.  Every member's dots with all of the node's (up to 14) pivot rows are
+// one tensor-core product, members x pivots, in f16 with fp32 accumulation:
+// codes are exact in f16 and every partial sum is an integer of magnitude <=
+// 2^24, so the dots are the exact int32 ones.  A warp takes 32 members (two
+// mma.m16n8k16 row tiles) against 16 columns; a lane reads 16 consecutive
+// codes of its rows (the K order is free as long as the pivots follow it) and
+// widens them in registers; the pivots are widened once per block into shared
+// memory, in the order the lanes read them.  Column 2j, 2j + 1 are the pivots
+// of descendant j, so lane c of a row holds both dots of descendants c and
+// 4 + c and decides their sides; the lanes exchange the seven bits and walk
+// the member's path.  side[e] = the member's path code; per tile and code the
+// member count, at bins[8*f + code*nt + (tile - f)] (f: the node's first tile,
+// nt: its tile count), so one exclusive scan of bins gives every member's
+// place.
+// Per member: d bytes of HBM (44 SM cycles at d = 1024), 52 instructions, 8
+// tensor instructions of 8 cycles, 2 shared-memory loads.  The dp4a form (the
+// member's own path only, 6 dots, 8 lanes per member) read 6 KB of pivot rows
+// from shared memory per member: 48 cycles that did not overlap the rows'
+// latency.  First round at 300k x 1024: 1.10 -> 0.77 ms (6.4 TB/s of rows, 0.94 of
+// the measured copy rate); all rounds at 1M 18.4 -> 13.5 ms.  Four CTAs per SM:
+// five spill (+15 %), three with a segment loaded ahead are 5 % slower.
+constexpr int kPivCols = 16;  // 14 pivots, two columns of zeros
+
+__device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {  // gram_tc.cu says how
+  const uint32_t u = w ^ 0x80808080u;
+  const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140);
+  const uint32_t b = __byte_perm(u, 0x64646464u, 0x4342);
+  asm("add.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(0xE480E480u));
+  asm("add.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(0xE480E480u));
+}
+
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__global__ void __launch_bounds__(256, 4) fuse_side(const int8_t* __restrict__ codes, int d,
+                                                    const int32_t* __restrict__ perm, NodeArr nd,
+                                                    const int32_t* __restrict__ tile_node,
+                                                    const int32_t* __restrict__ piv, uint8_t* __restrict__ side,
+                                                    int32_t* __restrict__ bins) {
+  // [d / 64][2 column tiles][2 halves][32 lanes] 16-byte pieces: lane (g, c) of
+  // column tile t finds pivot 8t + g's codes 16c..16c + 15 of the segment,
+  // widened, 8 in each half
+  extern __shared__ uint4 s_piv[];
+  __shared__ int32_t spv[kPivCols];
   __shared__ int32_t sbins[kFuseBins];
   const unsigned full = 0xffffffffu;
   const int b = blockIdx.x, tid = threadIdx.x;
   const int k = tile_node[b];
   if (tid < kFuseBins) sbins[tid] = 0;
-  if (tid < 2 * kFuseNodes) spv[tid] = piv[int64_t(k) * (2 * kFuseNodes) + tid];
+  if (tid < kPivCols) spv[tid] = tid < 2 * kFuseNodes ? piv[int64_t(k) * (2 * kFuseNodes) + tid] : -1;
   __syncthreads();
-  const int nchunk = d / 16;
-  for (int c = tid; c < 2 * kFuseNodes * nchunk; c += blockDim.x) {
-    const int r = c / nchunk, cc = c % nchunk;
+  const int nseg = d / 64;
+  for (int q = tid; q < kPivCols * 4 * nseg; q += 256) {
+    const int r = q / (4 * nseg), sc = q % (4 * nseg);  // pivot, 16-byte chunk of its row
     const int32_t id = spv[r];
-    if (id >= 0) prow[r][cc] = __ldg(reinterpret_cast<const uint4*>(codes + int64_t(id) * d) + cc);
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (id >= 0) v = __ldg(reinterpret_cast<const uint4*>(codes + int64_t(id) * d) + sc);
+    uint4 h0, h1;
+    widen4(v.x, h0.x, h0.y);
+    widen4(v.y, h0.z, h0.w);
+    widen4(v.z, h1.x, h1.y);
+    widen4(v.w, h1.z, h1.w);
+    uint4* dst = s_piv + ((sc >> 2) * 4 + (r >> 3) * 2) * 32 + (r & 7) * 4 + (sc & 3);
+    dst[0] = h0;
+    dst[32] = h1;
   }
   __syncthreads();
   const int32_t start = nd.start[k], size = nd.size[k];
   const int f = nd.p1[k], nt = (size + kTileElems - 1) / kTileElems;
   const int64_t e0 = int64_t(start) + int64_t(b - f) * kTileElems;
-  const int64_t e1 = min(int64_t(start) + size, e0 + kTileElems);
-  const int lane = tid & 31, warp = tid >> 5, sub = lane & 7, slot = lane >> 3;
-  const int per_lane = d / 128;
-  for (int step = 0; step < 8; ++step) {
-    const int t = warp * 32 + step * 4 + slot;
-    const int64_t e = e0 + t;
-    const bool valid = e < e1;
-    const int32_t id = valid ? perm[e] : -1;
-    uint4 v[kMaxDim / 128];
-    if (valid) {
-      const uint4* row = reinterpret_cast<const uint4*>(codes + int64_t(id) * d);
+  const int ne = int(min(int64_t(kTileElems), int64_t(start) + size - e0));  // members of this tile
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, c = lane & 3;
+  if (32 * warp < ne) {  // warp-uniform
+    // rows 8u + g of the warp's 32 members (past the end: the tile's last one)
+    int32_t id[4];
 #pragma unroll
-      for (int u = 0; u < kMaxDim / 128; ++u)
-        if (u < per_lane) v[u] = __ldg(row + sub + 8 * u);
+    for (int u = 0; u < 4; ++u) id[u] = perm[e0 + min(32 * warp + 8 * u + g, ne - 1)];
+    const int8_t* lane_codes = codes + 16 * c;
+    float acc[2][2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][t][e] = 0.f;
+#pragma unroll 1
+    for (int s = 0; s < nseg; ++s) {
+      uint4 raw[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        raw[u] = __ldg(reinterpret_cast<const uint4*>(lane_codes + int64_t(id[u]) * d + 64 * s));
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 b0 = s_piv[(s * 4 + h) * 32 + lane], b1 = s_piv[(s * 4 + 2 + h) * 32 + lane];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          uint32_t f0[4], f1[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            widen4(h == 0 ? (q == 0 ? raw[u].x : raw[u].y) : (q == 0 ? raw[u].z : raw[u].w), f0[u], f1[u]);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma16816(acc[m][0], f0[2 * m], f0[2 * m + 1], f1[2 * m], f1[2 * m + 1], q ? b0.z : b0.x, q ? b0.w : b0.y);
+            mma16816(acc[m][1], f0[2 * m], f0[2 * m + 1], f1[2 * m], f1[2 * m + 1], q ? b1.z : b1.x, q ? b1.w : b1.y);
+          }
+        }
+      }
     }
-    int j = 0, code = 0;
-    bool live = valid;
+    // bit j of byte u: member 8u + g's side at descendant j
+    uint32_t sides = 0;
 #pragma unroll
-    for (int dk = 0; dk < kFuse; ++dk) {
-      const int32_t p1 = live ? spv[2 * j] : -1, p2 = live ? spv[2 * j + 1] : -1;
-      const bool act = p1 >= 0;
-      int d1 = 0, d2 = 0;
-      if (act) {
-        d1 = dot_chunks(v, prow[2 * j], sub, per_lane);
-        d2 = dot_chunks(v, prow[2 * j + 1], sub, per_lane);
-      }
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int o = 1; o < 8; o <<= 1) {
-        d1 += __shfl_xor_sync(full, d1, o);
-        d2 += __shfl_xor_sync(full, d2, o);
+      for (int t = 0; t < 2; ++t) {
+        const int j = 4 * t + c;
+        const float d1 = acc[u >> 1][t][2 * (u & 1)], d2 = acc[u >> 1][t][2 * (u & 1) + 1];
+        const bool right = id[u] != spv[2 * j] && (id[u] == spv[2 * j + 1] || !(d1 > d2));
+        sides |= right ? 1u << (8 * u + j) : 0u;
       }
-      if (act) {
-        const int bit = id == p1 ? 0 : id == p2 ? 1 : (d1 > d2 ? 0 : 1);
-        code |= bit << (kFuse - 1 - dk);
-        j = 2 * j + 1 + bit;
-      } else {
-        live = false;
+    sides |= __shfl_xor_sync(full, sides, 1);
+    sides |= __shfl_xor_sync(full, sides, 2);
+    // lane c walks member 8c + g's path
+    const int x = 32 * warp + 8 * c + g;
+    if (x < ne) {
+      int j = 0, code = 0;
+#pragma unroll
+      for (int dk = 0; dk < kFuse; ++dk) {
+        if (j < kFuseNodes && spv[2 * j] >= 0) {
+          const int bit = int(sides >> (8 * c + j)) & 1;
+          code |= bit << (kFuse - 1 - dk);
+          j = 2 * j + 1 + bit;
+        } else {
+          j = kFuseNodes;  // not split below
+        }
       }
-    }
-    if (valid && sub == 0) {
-      side[e] = uint8_t(code);
+      side[e0 + x] = uint8_t(code);
       atomicAdd(&sbins[code], 1);
     }
   }
@@ -941,6 +996,8 @@ int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t 
     int32_t* tile_node = fb.child_cnt2;  // at most one tile per leaf_size + 1 members: fits
     int32_t host_cnt[3] = {0, 0, 0};
     int64_t tiles = int64_t(T) * root_tiles;
+    const size_t side_smem = size_t(kPivCols) * d * 2;
+    if ((e = ensure_smem_attr(reinterpret_cast<const void*>(fuse_side), side_smem))) return fail(e, "forest smem");
     if ((e = cudaMemsetAsync(fb.dev_i64, 0, 32, s))) return fail(e, "node counts");
     while (cnt > 0 && level < kMaxLevels) {
       if (tiles > fb.max_tiles || tiles > fb.max_nodes) {  // the tile -> node map has max_nodes entries
@@ -952,7 +1009,7 @@ int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t 
                                                 fb.max_nodes, fb.err, jt);
       note_launch();
       cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-      fuse_side<<<unsigned(tiles), 256, 0, s>>>(codes, d, perm, cur, tile_node, fb.piv, fb.side, fb.tile_bins);
+      fuse_side<<<unsigned(tiles), 256, side_smem, s>>>(codes, d, perm, cur, tile_node, fb.piv, fb.side, fb.tile_bins);
       note_launch();
       if ((e = exclusive_scan_i32(fb.tile_bins, fb.tile_bins_off, int64_t(kFuseBins) * tiles, nullptr, fb.scan_tmp, s)))
         return fail(e, "code scan");
