@@ -134,7 +134,7 @@ struct JoinLayout {
 __host__ __device__ constexpr uint32_t align16(uint32_t x) { return (x + 15u) & ~15u; }
 __host__ __device__ constexpr uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
-__host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d) {
+__host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool def) {
   JoinLayout s{};
   s.KK = K * K;
   s.pairs = (s.KK + 1) / 2;
@@ -147,11 +147,12 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d) {
     --s.ta_shift;
   }
   const uint32_t kk = uint32_t(2 * s.pairs), r = uint32_t(R);
-  s.dummy = align16(2 * kk) / 2;
+  // behind every occurrence index that a thread of the kernel forms
+  s.dummy = uint32_t(def ? (s.pairs + kThreads - 1) / kThreads : kMaxPairs) * kThreads * 2;
   uint32_t o = 0;
   s.o_ids = o;   o += align16(4 * kk);
   s.o_rep = o;   o += align16(umax(2 * kk, 14 * r));  // representatives, then the survivors' keys, ids and order
-  s.o_info = o;  o += align16(2 * kk) + 16;
+  s.o_info = o;  o += 2 * s.dummy + 16;
   s.o_ta = o;    o += uint32_t(s.ta_slots) * 4;
   s.o_tb = o;    o += kTableB * 4;
   s.o_hist = o;  o += kHBins * 4;  // also the row's cached distances, staged and gathered
@@ -217,13 +218,62 @@ __device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
 __device__ __forceinline__ void red_min(uint32_t a, uint32_t v) {
   asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
-__device__ __forceinline__ void red_min_if(bool p, uint32_t a, uint32_t v) {
-  asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q red.shared.min.u32 [%0], %1;\n}" ::"r"(a), "r"(v), "r"(uint32_t(p))
-               : "memory");
+// The table steps, each one piece so that its predicates stay predicates (a
+// C++ condition around an asm statement becomes a branch or a 0/1 register).
+// Insert: a candidate id (in range, not the row itself) writes `val` to its
+// slot and sets `bit`; any other id becomes kNone.
+__device__ __forceinline__ void table_insert(uint32_t& id, uint32_t n, uint32_t self, uint32_t slot, uint32_t val,
+                                             unsigned& valid, unsigned bit) {
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "setp.lt.u32 p, %0, %2;\n"
+      "setp.ne.and.u32 p, %0, %3, p;\n"
+      "@p red.shared.min.u32 [%4], %5;\n"
+      "@p or.b32 %1, %1, %6;\n"
+      "selp.b32 %0, %0, 0xffffffff, p;\n}"
+      : "+r"(id), "+r"(valid)
+      : "r"(n), "r"(self), "r"(slot), "r"(val), "r"(bit)
+      : "memory");
 }
-__device__ __forceinline__ void sts16_if(bool p, uint32_t a, uint32_t v) {
-  asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %2, 0;\n@q st.shared.u16 [%0], %1;\n}" ::"r"(a), "h"(uint16_t(v)), "r"(uint32_t(p))
-               : "memory");
+// Settle an occurrence j of `id` whose slot's winner w holds id `got`: a loser
+// enters the next round's table and sets its bit in `todo`; the winner itself
+// sets its bit in `first`.
+__device__ __forceinline__ void table_settle(uint32_t id, uint32_t got, uint32_t w, uint32_t j, uint32_t next_slot,
+                                             uint32_t next_val, unsigned& todo, unsigned& first, unsigned bit) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n"
+      "setp.ne.u32 p, %3, %2;\n"
+      "setp.ne.and.u32 p, %2, 0xffffffff, p;\n"
+      "@p red.shared.min.u32 [%6], %7;\n"
+      "@p or.b32 %0, %0, %8;\n"
+      "setp.eq.u32 q, %4, %5;\n"
+      "@q or.b32 %1, %1, %8;\n}"
+      : "+r"(todo), "+r"(first)
+      : "r"(id), "r"(got), "r"(w), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit)
+      : "memory");
+}
+// Look a cached id up in round 0: `e` is its slot, `base` the round's tag.  A
+// slot of an older round: absent.  Else the winner's id decides: equal, and the
+// cached info goes to the winner; other, and `bit` asks for the next round.
+__device__ __forceinline__ void table_find(uint32_t id, bool live, uint32_t e, uint32_t base, uint32_t a_ids, uint32_t a_info,
+                                           uint32_t info, unsigned& todo, unsigned bit) {
+  asm volatile(
+      "{\n.reg .pred p, q;\n.reg .b32 w, x, a;\n.reg .b16 h;\n"
+      "sub.u32 w, %2, %3;\n"
+      "setp.ne.u32 p, %7, 0;\n"
+      "setp.lt.and.u32 p, w, 4096, p;\n"
+      "mov.b32 x, 0xffffffff;\n"
+      "mad.lo.u32 a, w, 4, %4;\n"
+      "@p ld.shared.u32 x, [a];\n"
+      "setp.eq.and.u32 q, x, %1, p;\n"
+      "setp.ne.and.u32 p, x, %1, p;\n"
+      "mad.lo.u32 a, w, 2, %5;\n"
+      "cvt.u16.u32 h, %6;\n"
+      "@q st.shared.u16 [a], h;\n"
+      "@p or.b32 %0, %0, %8;\n}"
+      : "+r"(todo)
+      : "r"(id), "r"(e), "r"(base), "r"(a_ids), "r"(a_info), "r"(info), "r"(uint32_t(live)), "r"(bit)
+      : "memory");
 }
 __device__ __forceinline__ void red_add(uint32_t a, uint32_t v) {
   asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -311,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     counters += 8 * it;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl.times[2 * it] = global_ns();
   }
-  constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim);
+  constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim, true);
 #define KNNG_L(f) (DEF ? LD.f : LA.f)
   constexpr int NP = DEF ? (LD.pairs + kThreads - 1) / kThreads : kMaxPairs;  // pairs per thread
   const int K = DEF ? kDefK : K_, R = DEF ? kDefR : R_;
@@ -533,13 +583,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     for (int r = 0; r < NP; ++r) {
       const int p = tid + kThreads * r;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        uint32_t& id = v[2 * r + e];
-        const bool ok = id < n && id != uint32_t(i);
-        red_min_if(ok, a_ta + slot_of(id, 0u, KNNG_L(ta_shift)), tagj + uint32_t(2 * kThreads * r + e));
-        valid |= ok ? 1u << (2 * r + e) : 0u;
-        id = ok ? id : kNone;
-      }
+      for (int e = 0; e < 2; ++e)
+        table_insert(v[2 * r + e], n, uint32_t(i), a_ta + slot_of(v[2 * r + e], 0u, KNNG_L(ta_shift)),
+                     tagj + uint32_t(2 * kThreads * r + e), valid, 1u << (2 * r + e));
       if (p < KNNG_L(pairs)) sts64(a_ids + 8 * p, v[2 * r], v[2 * r + 1]);
     }
     {
@@ -565,11 +611,10 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         const int p = tid + kThreads * r;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          const uint32_t j = uint32_t(2 * p + e), id = v[2 * r + e];
-          const bool lost = lds32(a_ids + 4 * w[2 * r + e]) != id && id != kNone;
-          red_min_if(lost, a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e));
-          todo |= lost ? 1u << (2 * r + e) : 0u;
-          fm |= w[2 * r + e] == j && p < KNNG_L(pairs) ? 1u << (2 * r + e) : 0u;
+          const uint32_t id = v[2 * r + e];
+          table_settle(id, lds32(a_ids + 4 * w[2 * r + e]), w[2 * r + e], uint32_t(2 * p + e),
+                       a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e), todo,
+                       fm, 1u << (2 * r + e));
         }
         if (p < KNNG_L(pairs)) sts32(a_rep + 4 * p, w[2 * r] | (w[2 * r + 1] << 16));
       }
@@ -582,12 +627,8 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       const uint32_t hr = lds32(a_hist + 4 * q);
       const uint32_t e0 = lds32(a_ta + slot_of(id.x, 0u, KNNG_L(ta_shift)));
       const uint32_t e1 = lds32(a_ta + slot_of(id.y, 0u, KNNG_L(ta_shift)));
-      const uint32_t w0 = e0 & kJMask, w1 = e1 & kJMask;
-      const uint32_t x0 = lds32(a_ids + 4 * w0), x1 = lds32(a_ids + 4 * w1);
-      const bool t0 = 2 * q < cc && (e0 >> kJBits) == tag, t1 = 2 * q + 1 < cc && (e1 >> kJBits) == tag;
-      sts16_if(t0 && x0 == id.x, a_info + 2 * w0, hr | kKnown);
-      sts16_if(t1 && x1 == id.y, a_info + 2 * w1, (hr >> 16) | kKnown);
-      ctodo |= (t0 && x0 != id.x ? 1u << (2 * u) : 0u) | (t1 && x1 != id.y ? 2u << (2 * u) : 0u);
+      table_find(id.x, 2 * q < cc, e0, tag << kJBits, a_ids, a_info, hr | kKnown, ctodo, 1u << (2 * u));
+      table_find(id.y, 2 * q + 1 < cc, e1, tag << kJBits, a_ids, a_info, (hr >> 16) | kKnown, ctodo, 2u << (2 * u));
     }
     if (find_id != ~0u) {
       const uint32_t e = lds32(a_ta + slot_of(find_id, 0u, KNNG_L(ta_shift)));
@@ -767,9 +808,10 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
 #pragma unroll 1
       for (int base = 0; base < kHBins; base += 128) {
         const uint4 b4 = lds128(a_hist + 4 * (base + 4 * lane));
-        const int sum = int(b4.x + b4.y + b4.z + b4.w), incl = warp_incl_scan(sum, lane);
-        const int tot = __shfl_sync(full, incl, 31);
+        const int sum = int(b4.x + b4.y + b4.z + b4.w);
+        const int tot = __reduce_add_sync(full, sum);
         if (acc + tot >= R) {  // warp-uniform; reached, as the bins hold cnt > R occurrences
+          const int incl = warp_incl_scan(sum, lane);
           int run = acc + incl - sum, x = base + 4 * lane;
           const bool here = run < R && R <= run + sum;
           if (run + int(b4.x) < R) {
@@ -1121,7 +1163,7 @@ JoinKernel pick_variant(int ctas_per_sm, int cblock) {
 // their own kernel, which reads the lists 8 bytes at a time (`aligned`).
 JoinKernel variant(int K, int R, int d, bool aligned, int ctas_per_sm, int cblock, JoinLayout* L) {
   const bool def = K == kDefK && R == kDefR && aligned;
-  *L = join_layout(K, R, def ? kMaxDim : d);
+  *L = join_layout(K, R, def ? kMaxDim : d, def);
   return def ? pick_variant<true>(ctas_per_sm, cblock) : pick_variant<false>(ctas_per_sm, cblock);
 }
 
