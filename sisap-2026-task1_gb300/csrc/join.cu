@@ -161,7 +161,7 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
   s.o_x = o;     o += align16(umax(umax(kCacheCap * 4, uint32_t((s.pairs + kThreads - 1) / kThreads) * kThreads * 4), 2 * r));
   s.o_pool = o;  o += 2 * 2 * kMaxK * 4;  // starting lists of this row and of the previous one: ids, scores
   s.o_row = o;   o += 2 * 32;             // row counters, by row parity
-  s.o_cell = o;  o += kMaxPairs * kWarps * 4;  // threshold ties per (round, warp)
+  s.o_cell = o;  o += align16(kMaxPairs * kWarps * 4);  // threshold ties per (round, warp)
   s.o_sk = o;    o += 128;                // the widest sketch
   s.o_code = o;  o += align16(uint32_t(d));
   s.bytes = o;
