@@ -73,8 +73,8 @@
 //      R - count(h > h_t) occurrences with h == h_t in j order, ranked by
 //      ballot counts per (round, warp); the selected first occurrences that
 //      are neither starting-list members nor known to be rejected need a dot
-//   F  dp4a dots, 8 lanes per candidate; keep those above the starting
-//      pool[K-1].score, flag the others as rejected
+//   F  dp4a dots, a warp per four candidates (short rows: 8 lanes each); keep
+//      those above the starting pool[K-1].score, flag the others as rejected
 //   G  write the row's cache (this iteration's distinct ids, h and flags);
 //      insertion by rank counting over 64-bit survivor keys {dot, visit key}
 //      (or the reference's sequential loop for an unsorted or unscored pool),
@@ -309,17 +309,104 @@ __device__ __forceinline__ int dot_u4(uint4 a, uint4 b, int acc) {
   return __dp4a(int(a.w), int(b.w), acc);
 }
 
-// A lane's share of the dot of a code row (its 16-byte chunks 128 bytes apart
-// from `row` on) with the row in shared memory.
+// What stage F does with a candidate's dot: above the starting threshold it is
+// a survivor, else (with a candidate cache) flagged as rejected.
+struct DotSink {
+  uint32_t a_row, a_need, a_ids, a_info, a_thr, a_key, a_sid;
+  bool flag_rejected;
+  __device__ __forceinline__ void take(int q, int dot) const {
+    const uint32_t j = lds16(a_need + 2 * q), f = lds16(a_info + 2 * j);
+    if (dot > int32_t(lds32(a_thr))) {
+      const uint32_t at = atom_add(a_row + kRowProm, 1u);
+      sts64(a_key + 8 * at, ((1024u - (f & kXMask)) << 13) | (0x1fffu - j), uint32_t(dot) ^ 0x80000000u);
+      sts32(a_sid + 4 * at, lds32(a_ids + 4 * j));
+    } else if (flag_rejected) {
+      sts16(a_info + 2 * j, f | kRej);
+    }
+  }
+};
+
+// Stage F for rows of 257 to 512 * HALVES codes: a warp per four candidates, a
+// lane the 16-byte chunks lane and lane + 32 of each, so the row's own chunks
+// stay in registers.  (With 8 lanes per candidate they were read from shared
+// memory for every candidate, four wavefronts per load like the gather itself.)
+// The four sums are reduced together: each exchange keeps half of them.
+template <int HALVES>
+__device__ __forceinline__ void dots_wide(const int8_t* __restrict__ codes, int d, uint32_t self, uint32_t a_code, int tid,
+                                          const DotSink& sink) {
+  const unsigned full = 0xffffffffu;
+  const int lane = tid & 31;
+  const int nneed = int(lds32(sink.a_row + kRowNeed));
+  int b = 4 * (tid >> 5);
+  if (b >= nneed) return;  // warp-uniform
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  bool live[HALVES];
+  uint4 mine[HALVES];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h) {
+    live[h] = 512 * h + 16 * lane < d;
+    mine[h] = live[h] ? lds128(a_code + 512 * h + 16 * lane) : zero;
+  }
+  const int8_t* lane_codes = codes + 16 * lane;
+#pragma unroll 1
+  for (; b < nneed; b += 4 * kWarps) {
+    const uint2 list = lds64(sink.a_need + 2 * b);  // four entries; the row itself past the list's end
+    uint4 x[4][HALVES];
+    int acc[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t j = ((c < 2 ? list.x : list.y) >> (16 * (c & 1))) & 0xffffu;
+      const uint32_t id = b + c < nneed ? lds32(sink.a_ids + 4 * j) : self;
+      const int8_t* row = lane_codes + uint64_t(id) * uint32_t(d);
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        x[c][h] = zero;
+        if (live[h]) x[c][h] = __ldg(reinterpret_cast<const uint4*>(row + 512 * h));
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      acc[c] = 0;
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) acc[c] = dot_u4(x[c][h], mine[h], acc[c]);
+    }
+    const bool hi = lane & 16, mid = lane & 8;
+    int k0 = hi ? acc[2] : acc[0], k1 = hi ? acc[3] : acc[1];
+    k0 += __shfl_xor_sync(full, hi ? acc[0] : acc[2], 16);
+    k1 += __shfl_xor_sync(full, hi ? acc[1] : acc[3], 16);
+    int k = mid ? k1 : k0;
+    k += __shfl_xor_sync(full, mid ? k0 : k1, 8);
+    k += __shfl_xor_sync(full, k, 4);
+    k += __shfl_xor_sync(full, k, 2);
+    k += __shfl_xor_sync(full, k, 1);
+    const int q = b + (lane >> 3);  // lanes 8c..8c + 7 hold candidate c's sum
+    if ((lane & 7) == 0 && q < nneed) sink.take(q, k);
+  }
+}
+
+// Stage F for short rows: 8 lanes per candidate, 128 * CHUNKS codes.
 template <int CHUNKS>
-__device__ __forceinline__ int dot_lane(const int8_t* row, uint32_t mine) {
-  uint4 x[CHUNKS];
-  int acc = 0;
+__device__ __forceinline__ void dots_narrow(const int8_t* __restrict__ codes, uint32_t a_code, int tid, const DotSink& sink) {
+  const unsigned full = 0xffffffffu;
+  const int sub = tid & 7, slot8 = (tid & 31) >> 3;
+  const int nneed = int(lds32(sink.a_row + kRowNeed));
+#pragma unroll 1
+  for (int q = tid >> 3; q - slot8 < nneed; q += kGroups) {
+    int acc = 0;
+    if (q < nneed) {
+      const uint32_t id = lds32(sink.a_ids + 4 * lds16(sink.a_need + 2 * q));
+      const int8_t* row = codes + uint64_t(id) * uint32_t(128 * CHUNKS) + 16 * sub;
+      uint4 x[CHUNKS];
 #pragma unroll
-  for (int u = 0; u < CHUNKS; ++u) x[u] = __ldg(reinterpret_cast<const uint4*>(row + 128 * u));
+      for (int u = 0; u < CHUNKS; ++u) x[u] = __ldg(reinterpret_cast<const uint4*>(row + 128 * u));
 #pragma unroll
-  for (int u = 0; u < CHUNKS; ++u) acc = dot_u4(x[u], lds128(mine + 128 * u), acc);
-  return acc;
+      for (int u = 0; u < CHUNKS; ++u) acc = dot_u4(x[u], lds128(a_code + 16 * sub + 128 * u), acc);
+    }
+    acc += __shfl_xor_sync(full, acc, 1);
+    acc += __shfl_xor_sync(full, acc, 2);
+    acc += __shfl_xor_sync(full, acc, 4);
+    if (sub == 0 && q < nneed) sink.take(q, acc);
+  }
 }
 
 // Byte offset of id's slot in a table of 2^(32 - shift) words, round 0 or
@@ -897,42 +984,13 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       }
     }
     __syncthreads();
-    // ---- F  dots (8 lanes per candidate, up to eight 16-byte loads in flight per lane)
+    // ---- F  dots
     {
-      const int per_lane = d / 128;
-#pragma unroll 1
-      for (int q = warp * 4 + slot8; q - slot8 < int(lds32(a_row + kRowNeed)); q += kGroups) {
-        const bool live = q < int(lds32(a_row + kRowNeed));
-        int acc = 0;
-        if (live) {
-          const uint32_t id = lds32(a_ids + 4 * lds16(a_x + 2 * q));
-          const int8_t* row = codes + int64_t(id) * d + 16 * sub;
-          const uint32_t mine = a_code + 16 * sub;
-          switch (per_lane) {  // uniform; one body per width, so that all its loads are in flight without predicates
-            case 1: acc = dot_lane<1>(row, mine); break;
-            case 2: acc = dot_lane<2>(row, mine); break;
-            case 3: acc = dot_lane<3>(row, mine); break;
-            case 4: acc = dot_lane<4>(row, mine); break;
-            case 5: acc = dot_lane<5>(row, mine); break;
-            case 6: acc = dot_lane<6>(row, mine); break;
-            case 7: acc = dot_lane<7>(row, mine); break;
-            default: acc = dot_lane<8>(row, mine); break;
-          }
-        }
-        acc += __shfl_xor_sync(full, acc, 1);
-        acc += __shfl_xor_sync(full, acc, 2);
-        acc += __shfl_xor_sync(full, acc, 4);
-        if (sub == 0 && live) {
-          const uint32_t j = lds16(a_x + 2 * q), id = lds32(a_ids + 4 * j), f = lds16(a_info + 2 * j);
-          if (acc > int32_t(lds32(a_psc + 4 * (K - 1)))) {
-            const uint32_t at = atom_add(a_row + kRowProm, 1u);
-            sts64(a_rep + 8 * at, ((1024u - (f & kXMask)) << 13) | (0x1fffu - j), uint32_t(acc) ^ 0x80000000u);
-            sts32(a_sid + 4 * at, id);
-          } else if (cached) {
-            sts16(a_info + 2 * j, f | kRej);
-          }
-        }
-      }
+      const DotSink sink{a_row, a_x, a_ids, a_info, a_psc + 4 * (K - 1), a_rep, a_sid, cached};
+      if (d > 512) dots_wide<2>(codes, d, uint32_t(i), a_code, tid, sink);  // uniform
+      else if (d > 256) dots_wide<1>(codes, d, uint32_t(i), a_code, tid, sink);
+      else if (d > 128) dots_narrow<2>(codes, a_code, tid, sink);
+      else dots_narrow<1>(codes, a_code, tid, sink);
     }
     __syncthreads();
     // ---- G  the row's cache for the next iteration: this iteration's distinct
