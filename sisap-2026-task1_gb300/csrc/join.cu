@@ -114,7 +114,6 @@ constexpr uint32_t kXMask = 0x7ffu;          // info bits 0..10: Hamming distanc
 constexpr uint32_t kKnown = 0x800u;          // info bit 11: distance taken from the row's candidate cache
 constexpr uint32_t kRej = 0x1000u;           // info bit 12: dot known to be <= the row's pool threshold
 constexpr uint32_t kNone = 0xffffffffu;      // ids: no candidate (no id equals it: num_trees * n < 2^31)
-constexpr uint32_t kPoolFlag = 0x80000000u;  // ids bit 31: the id is in the starting list with a real score
 // The default parameters get a kernel of their own whose sizes and
 // shared-memory offsets are compile-time constants: read from the parameter
 // block they cost about 4,000 more instructions per row.
@@ -127,7 +126,7 @@ struct JoinLayout {
   int ta_slots, ta_shift;  // first table: slots and hash shift
   uint32_t kdiv;           // j / K = (j * kdiv) >> 20 for j < 4096
   uint32_t dummy;          // info index of occurrences without a candidate
-  uint32_t o_code, o_sk, o_ids, o_rep, o_info, o_ta, o_tb, o_hist, o_x, o_pool, o_row, o_cell;
+  uint32_t o_code, o_sk, o_ids, o_rep, o_info, o_ta, o_tb, o_hist, o_x, o_pool, o_row, o_cell, o_member;
   uint32_t bytes;
 };
 
@@ -162,6 +161,7 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
   s.o_pool = o;  o += 2 * 2 * kMaxK * 4;  // starting lists of this row and of the previous one: ids, scores
   s.o_row = o;   o += 2 * 32;             // row counters, by row parity
   s.o_cell = o;  o += align16(kMaxPairs * kWarps * 4);  // threshold ties per (round, warp)
+  s.o_member = o; o += kThreads * 4;      // per thread: its occurrences whose id is in the starting list
   s.o_sk = o;    o += 128;                // the widest sketch
   s.o_code = o;  o += align16(uint32_t(d));
   s.bytes = o;
@@ -238,18 +238,19 @@ __device__ __forceinline__ void table_insert(uint32_t& id, uint32_t n, uint32_t 
 // Settle an occurrence j of `id` whose slot's winner w holds id `got`: a loser
 // enters the next round's table and sets its bit in `todo`; the winner itself
 // sets its bit in `first`.
-__device__ __forceinline__ void table_settle(uint32_t id, uint32_t got, uint32_t w, uint32_t j, uint32_t next_slot,
+__device__ __forceinline__ void table_settle(uint32_t id, uint32_t got, uint32_t& w, uint32_t dummy, uint32_t j, uint32_t next_slot,
                                              uint32_t next_val, unsigned& todo, unsigned& first, unsigned bit) {
   asm volatile(
       "{\n.reg .pred p, q;\n"
-      "setp.ne.u32 p, %3, %2;\n"
-      "setp.ne.and.u32 p, %2, 0xffffffff, p;\n"
-      "@p red.shared.min.u32 [%6], %7;\n"
-      "@p or.b32 %0, %0, %8;\n"
-      "setp.eq.u32 q, %4, %5;\n"
-      "@q or.b32 %1, %1, %8;\n}"
-      : "+r"(todo), "+r"(first)
-      : "r"(id), "r"(got), "r"(w), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit)
+      "setp.ne.u32 q, %3, 0xffffffff;\n"
+      "selp.b32 %2, %2, %5, q;\n"
+      "setp.ne.and.u32 p, %4, %3, q;\n"
+      "@p red.shared.min.u32 [%7], %8;\n"
+      "@p or.b32 %0, %0, %9;\n"
+      "setp.eq.u32 q, %2, %6;\n"
+      "@q or.b32 %1, %1, %9;\n}"
+      : "+r"(todo), "+r"(first), "+r"(w)
+      : "r"(id), "r"(got), "r"(dummy), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit)
       : "memory");
 }
 // Look a cached id up in round 0: `e` is its slot, `base` the round's tag.  A
@@ -274,6 +275,52 @@ __device__ __forceinline__ void table_find(uint32_t id, bool live, uint32_t e, u
       : "+r"(todo)
       : "r"(id), "r"(e), "r"(base), "r"(a_ids), "r"(a_info), "r"(info), "r"(uint32_t(live)), "r"(bit)
       : "memory");
+}
+// Threshold step of stage E: `bit` goes to `near` if key < xt, to `at` if dist == xt, to `open` if key == xt.
+__device__ __forceinline__ void mark_near(uint32_t key, uint32_t dist, uint32_t xt, unsigned& near, unsigned& at,
+                                          unsigned& open, unsigned bit) {
+  asm("{\n.reg .pred p, q, t;\n"
+      "setp.lt.u32 p, %3, %5;\n"
+      "setp.eq.u32 q, %4, %5;\n"
+      "setp.eq.u32 t, %3, %5;\n"
+      "@p or.b32 %0, %0, %6;\n"
+      "@q or.b32 %1, %1, %6;\n"
+      "@t or.b32 %2, %2, %6;\n}"
+      : "+r"(near), "+r"(at), "+r"(open)
+      : "r"(key), "r"(dist), "r"(xt), "r"(bit));
+}
+// If `bit` of `m` is set: store the half word at `at` and step on.
+__device__ __forceinline__ void list_push(unsigned m, unsigned bit, uint32_t& at, uint32_t val) {
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b32 t;\n.reg .b16 h;\n"
+      "and.b32 t, %1, %2;\n"
+      "setp.ne.u32 p, t, 0;\n"
+      "cvt.u16.u32 h, %3;\n"
+      "@p st.shared.u16 [%0], h;\n"
+      "@p add.u32 %0, %0, 2;\n}"
+      : "+r"(at)
+      : "r"(m), "r"(bit), "r"(val)
+      : "memory");
+}
+// The same for an entry of a row's next cache: id and info word, while at < end.
+__device__ __forceinline__ void cache_push(unsigned m, unsigned bit, uint32_t& at_id, uint32_t& at_info, uint32_t end,
+                                           uint32_t id, uint32_t info) {
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b32 t;\n.reg .b16 h;\n"
+      "and.b32 t, %2, %3;\n"
+      "setp.ne.u32 p, t, 0;\n"
+      "setp.lt.and.u32 p, %0, %4, p;\n"
+      "cvt.u16.u32 h, %6;\n"
+      "@p st.shared.u32 [%0], %5;\n"
+      "@p st.shared.u16 [%1], h;\n"
+      "@p add.u32 %0, %0, 4;\n"
+      "@p add.u32 %1, %1, 2;\n}"
+      : "+r"(at_id), "+r"(at_info)
+      : "r"(m), "r"(bit), "r"(end), "r"(id), "r"(info)
+      : "memory");
+}
+__device__ __forceinline__ void red_or(uint32_t a, uint32_t v) {
+  asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 __device__ __forceinline__ void red_add(uint32_t a, uint32_t v) {
   asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -466,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
   const uint32_t a_ids = sb + KNNG_L(o_ids), a_rep = sb + KNNG_L(o_rep), a_info = sb + KNNG_L(o_info);
   const uint32_t a_ta = sb + KNNG_L(o_ta), a_tb = sb + KNNG_L(o_tb), a_hist = sb + KNNG_L(o_hist);
   const uint32_t a_x = sb + KNNG_L(o_x), a_cell = sb + KNNG_L(o_cell), a_code = sb + KNNG_L(o_code);
+  const uint32_t a_member = sb + KNNG_L(o_member);
   // survivors: 64-bit keys {dot, visit key}, then ids, then (sequential insertion) their visit order
   const uint32_t a_sid = a_rep + 8u * uint32_t(R), a_sorder = a_rep + 12u * uint32_t(R);
   // per-CTA statistics, kept by thread 0 in shared memory (no registers held
@@ -491,6 +539,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     for (int t = tid; t < kTableB / 4; t += kThreads) sts128(a_tb + 16 * t, e);
   };
   clear_tables();
+  sts32(a_member + 4 * tid, 0);
   uint32_t tag = kTagTop;           // block-uniform
   uint32_t par = 0;                 // parity of the computed rows
 
@@ -665,13 +714,16 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     // a valid id goes into the first table; without a candidate the register
     // holds kNone, which no id in shared memory equals
     unsigned valid = 0;  // bit 2r + e
+    uint32_t sl[2 * NP];
+#pragma unroll
+    for (int x = 0; x < 2 * NP; ++x) sl[x] = a_ta + slot_of(v[x], 0u, KNNG_L(ta_shift));
     const uint32_t tagj = (tag << kJBits) + 2u * uint32_t(tid);
 #pragma unroll
     for (int r = 0; r < NP; ++r) {
       const int p = tid + kThreads * r;
 #pragma unroll
       for (int e = 0; e < 2; ++e)
-        table_insert(v[2 * r + e], n, uint32_t(i), a_ta + slot_of(v[2 * r + e], 0u, KNNG_L(ta_shift)),
+        table_insert(v[2 * r + e], n, uint32_t(i), sl[2 * r + e],
                      tagj + uint32_t(2 * kThreads * r + e), valid, 1u << (2 * r + e));
       if (p < KNNG_L(pairs)) sts64(a_ids + 8 * p, v[2 * r], v[2 * r + 1]);
     }
@@ -690,8 +742,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       uint32_t w[2 * NP];
 #pragma unroll
       for (int x = 0; x < 2 * NP; ++x) {
-        w[x] = lds32(a_ta + slot_of(v[x], 0u, KNNG_L(ta_shift))) & kJMask;
-        w[x] = v[x] == kNone ? KNNG_L(dummy) : w[x];
+        w[x] = lds32(sl[x]) & kJMask;
       }
 #pragma unroll
       for (int r = 0; r < NP; ++r) {
@@ -699,7 +750,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const uint32_t id = v[2 * r + e];
-          table_settle(id, lds32(a_ids + 4 * w[2 * r + e]), w[2 * r + e], uint32_t(2 * p + e),
+          table_settle(id, lds32(a_ids + 4 * w[2 * r + e]), w[2 * r + e], KNNG_L(dummy), uint32_t(2 * p + e),
                        a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e), todo,
                        fm, 1u << (2 * r + e));
         }
@@ -776,7 +827,10 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     // ---- C  Hamming once per distinct id without a cached distance: each warp
     //         lists its own first occurrences that are misses and scores them
     //         (groups of 8 lanes, CB candidates in flight per group)
-    if (find_rep >= 0) sts32(a_ids + 4 * find_rep, lds32(a_ids + 4 * find_rep) | kPoolFlag);
+    if (find_rep >= 0) {  // occurrence 2 (t + 256 r) + e: bit 2r + e of thread t's word
+      const uint32_t p = uint32_t(find_rep) >> 1;
+      red_or(a_member + 4 * (p % kThreads), 1u << (2 * (p / kThreads) + (uint32_t(find_rep) & 1u)));
+    }
     for (int t = tid; t < kHBins / 4; t += kThreads) sts128(a_hist + 16 * t, make_uint4(0, 0, 0, 0));
     int first_at;  // this thread's place among the row's distinct ids (stage G)
     {
@@ -792,9 +846,10 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
           }
         }
       }
-      const int c = __popc(mm), incl = warp_incl_scan(c, lane);
+      const int c = __popc(mm), nfirst = __popc(fm);
+      const int both = warp_incl_scan(c | (nfirst << 16), lane);  // two sums, at most 32 * 2 NP each
+      const int incl = both & 0xffff, fincl = both >> 16;
       const int nm = __shfl_sync(full, incl, 31);
-      const int nfirst = __popc(fm), fincl = warp_incl_scan(nfirst, lane);
       int wbase = 0;
       if (lane == 31) {
         wbase = int(atom_add(a_row + kRowNu, uint32_t(fincl)));
@@ -804,11 +859,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       // up to 64 NP misses per warp
       const uint32_t a_miss = a_x + uint32_t(warp) * (DEF ? uint32_t(NP) * 128u : uint32_t((LA.pairs + kThreads - 1) / kThreads) * 128u);
       uint32_t at = a_miss + 2 * (incl - c);
-#pragma unroll 1
-      for (; mm; mm &= mm - 1u, at += 2) {
-        const int b = __ffs(mm) - 1;
-        sts16(at, 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1));
-      }
+      const uint32_t j0 = 2u * uint32_t(tid);
+#pragma unroll
+      for (int b = 0; b < 2 * NP; ++b) list_push(mm, 1u << b, at, j0 + uint32_t(2 * kThreads * (b >> 1) + (b & 1)));
       __syncwarp();
       const char* sk_base = reinterpret_cast<const char*>(sketch);
       const uint32_t sk_bytes = uint32_t(W) * 8u;
@@ -816,7 +869,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         const uint4 mine = lds128(sb + KNNG_L(o_sk));
 #pragma unroll 1
         for (int q = lane; q < nm; q += 32) {
-          const uint32_t j = lds16(a_miss + 2 * q), id = lds32(a_ids + 4 * j) & ~kPoolFlag;
+          const uint32_t j = lds16(a_miss + 2 * q), id = lds32(a_ids + 4 * j);
           sts16(a_info + 2 * j, popc_u4(__ldg(reinterpret_cast<const uint4*>(sk_base + uint64_t(id) * 16u)), mine));
         }
       } else {
@@ -835,7 +888,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
           uint32_t j = 0, id = uint32_t(i);  // past the list: the row itself
           if (q < nm) {
             j = lds16(a_miss + 2 * q);
-            id = lds32(a_ids + 4 * j) & ~kPoolFlag;
+            id = lds32(a_ids + 4 * j);
           }
           uint32_t pw[4] = {0, 0, 0, 0};  // word k: candidates u = k (low half) and u = k + 4
 #pragma unroll
@@ -926,16 +979,17 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     //         selected iff fewer than need_eq ties come before it in j order
     //         (a cached rejection stands: the row's threshold never falls, so
     //         a dot once <= it stays <= it)
-    unsigned wm = 0, eqm = 0;  // nearer than the threshold; at it
+    unsigned wm = 0, eqm = 0, open = 0;  // nearer than the threshold; at it; at it and not rejected
 #pragma unroll
     for (int r = 0; r < NP; ++r) {
-      const uint32_t x0 = hv[r] & kXMask, x1 = (hv[r] >> 16) & kXMask;
-      if (x0 < xt && !(hv[r] & kRej)) wm |= 1u << (2 * r);
-      if (x1 < xt && !(hv[r] & (kRej << 16))) wm |= 2u << (2 * r);
-      if (x0 == xt) eqm |= 1u << (2 * r);
-      if (x1 == xt) eqm |= 2u << (2 * r);
+      // a rejection's bit lies above the distance: such a word is never below xt
+      mark_near(hv[r] & (kXMask | kRej), hv[r] & kXMask, xt, wm, eqm, open, 1u << (2 * r));
+      mark_near(hv[r] & ((kXMask | kRej) << 16), hv[r] & (kXMask << 16), xt << 16, wm, eqm, open, 2u << (2 * r));
     }
-    wm &= fm;
+    const unsigned want = fm & ~lds32(a_member + 4 * tid);
+    sts32(a_member + 4 * tid, 0);
+    wm &= want;
+    open &= want;
     if (cut) {
       // ties per (round, warp): j ascends with round, warp, lane, element
       const unsigned any = __reduce_or_sync(full, eqm);
@@ -948,29 +1002,25 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         if (lane == 0) sts32(a_cell + 4 * (r * kWarps + warp), uint32_t(c));
       }
       __syncthreads();
-      if (any) {  // warp-uniform
+      const unsigned decide = __reduce_or_sync(full, open);
+      if (decide) {  // warp-uniform
         uint2 c2 = make_uint2(0, 0);
         if (2 * lane < NP * kWarps) c2 = lds64(a_cell + 8 * lane);
         const int sum = int(c2.x + c2.y);
         const int pre = warp_incl_scan(sum, lane) - sum + ((warp & 1) ? int(c2.x) : 0);
 #pragma unroll
         for (int r = 0; r < NP; ++r) {
-          if ((any >> (2 * r)) & 3u) {  // warp-uniform
+          if ((decide >> (2 * r)) & 3u) {  // warp-uniform
             const unsigned b0 = __ballot_sync(full, (eqm >> (2 * r)) & 1u), b1 = __ballot_sync(full, (eqm >> (2 * r)) & 2u);
             const int before = __shfl_sync(full, pre, 4 * r + (warp >> 1)) + __popc(b0 & lt) + __popc(b1 & lt);
             const unsigned e0 = (eqm >> (2 * r)) & 1u;
-            if (e0 && before < need_eq && !(hv[r] & kRej)) wm |= (1u << (2 * r)) & fm;
-            if (((eqm >> (2 * r)) & 2u) && before + int(e0) < need_eq && !(hv[r] & (kRej << 16))) wm |= (2u << (2 * r)) & fm;
+            if (before < need_eq) wm |= open & (1u << (2 * r));
+            if (before + int(e0) < need_eq) wm |= open & (2u << (2 * r));
           }
         }
       }
     }
     {
-#pragma unroll 1
-      for (unsigned m = wm; m; m &= m - 1u) {
-        const int b = __ffs(m) - 1;
-        if (int32_t(lds32(a_ids + 8 * (tid + kThreads * (b >> 1)) + 4 * (b & 1))) < 0) wm ^= 1u << b;
-      }
       if (__any_sync(full, wm != 0)) {
         const int c = __popc(wm), incl = warp_incl_scan(c, lane);
         uint32_t base = 0;
@@ -998,14 +1048,17 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     //         gathered in shared memory (over the rerank list and the
     //         histogram) and written out 16 bytes at a time below
     if (cached) {
-#pragma unroll 1
-      for (unsigned m = fm; m; m &= m - 1u, ++first_at) {
-        if (first_at >= ctl.cache_cap) break;
-        const int b = __ffs(m) - 1;
-        const uint32_t j = 2u * uint32_t(tid + kThreads * (b >> 1)) + uint32_t(b & 1);
-        const uint32_t id = lds32(a_ids + 4 * j), f = lds16(a_info + 2 * j);
-        sts32(a_x + 4 * first_at, id & ~kPoolFlag);
-        sts16(a_hist + 2 * first_at, f & ~kKnown);
+      uint32_t at_id = a_x + 4u * uint32_t(first_at), at_info = a_hist + 2u * uint32_t(first_at);
+      const uint32_t end = a_x + 4u * uint32_t(ctl.cache_cap);
+#pragma unroll
+      for (int r = 0; r < NP; ++r) {
+        const int p = tid + kThreads * r;
+        if (p < KNNG_L(pairs)) {
+          const uint2 id = lds64(a_ids + 8 * p);
+          const uint32_t f = lds32(a_info + 4 * p) & ~(kKnown | (kKnown << 16));
+          cache_push(fm, 1u << (2 * r), at_id, at_info, end, id.x, f);
+          cache_push(fm, 2u << (2 * r), at_id, at_info, end, id.y, f >> 16);
+        }
       }
     }
     //         insertion of the survivors in visit order.  The pool's last score
