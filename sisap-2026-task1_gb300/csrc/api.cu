@@ -80,11 +80,15 @@ struct DevBuf {
   }
 };
 
-// (ctas_per_sm, cblock) of the join for its first two iterations, where most
-// candidates are new, and for the later ones, where the candidate cache serves
-// most of them: the two favour different occupancy/in-flight trade-offs.
+// The join's form (ctas_per_sm, cblock, far) for its first two iterations,
+// where most candidates are new, and for the later ones, where the candidate
+// cache serves most of them: the two favour different trade-offs.
+struct JoinForm {
+  int ctas = 4, cblock = 4;
+  bool far = false;
+};
 struct JoinCfg {
-  std::pair<int, int> early{4, 4}, late{4, 4};
+  JoinForm early, late;
 };
 
 struct knng_ctx {
@@ -125,7 +129,10 @@ struct knng_ctx {
 
 namespace {
 
-constexpr int kTuneReps = 2;  // timed launches per configuration of an autotune sweep (the faster one counts)
+// Timed launches per configuration of an autotune sweep (the fastest counts).
+// The early iterations take most of the phase and their configurations lie
+// closest together, so theirs gets one more.
+constexpr int kEarlyReps = 3, kLateReps = 2;
 constexpr int64_t kStageRows = 1 << 16;  // host-input rows per H2D chunk (256 MB at d = 1024)
 // byte offset in the context's 4096-byte scalar block of the bounds-checked
 // build's error word (the forest uses bytes 0..67, the initial graph 128..159,
@@ -338,9 +345,13 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   const knng_params& p = c->prm;
   JoinCfg best;
   if (p.join_ctas_per_sm) {  // a forced variant
-    best.early = best.late = std::make_pair(p.join_ctas_per_sm, p.join_cblock);
+    best.early = best.late = JoinForm{p.join_ctas_per_sm, p.join_cblock, false};
     return best;
   }
+  // Rows from beyond L2: a sweep over part of the rows would find them in L2,
+  // so the early form's far flag is not left to it.
+  const bool far_early = join_far(N, d) && join_has_far(p.k_build, p.k_build * p.rerank_mult);
+  best.early.far = far_early;
   const auto key = std::make_pair(d, int(std::log2(double(N))));
   auto it = c->tuned.find(key);
   if (it != c->tuned.end()) return it->second;
@@ -349,7 +360,12 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
     c->last_error = std::string("join variants: ") + join_variant_error();
     return best;
   }
-  const std::pair<int, int> cand[] = {{4, 4}, {4, 8}, {3, 4}, {3, 8}, {4, 2}};
+  // With a far form three CTAs are never the fastest: 300,000 x 1024 of
+  // 64-dimensional data, join of two iterations: 4 CTAs 62.7 ms, 3 CTAs 49.9,
+  // 4 far CTAs 45.5; 600,000 x 1024 clustered, first iteration: 33.7, 31.0, 28.7.
+  const JoinForm with_far[] = {{4, 4, false}, {4, 8, false}, {4, 4, true}, {4, 8, true}, {4, 2, false}};
+  const JoinForm general[] = {{4, 4, false}, {4, 8, false}, {3, 4, false}, {3, 8, false}, {4, 2, false}};
+  const auto& cand = join_has_far(p.k_build, p.k_build * p.rerank_mult) ? with_far : general;
   const int K = p.k_build;
   // the sweeps process the first 1/16 of the rows (at least 64 per resident CTA),
   // so tuning costs about one join launch on the first build of a bucket
@@ -357,14 +373,15 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   plain.row_limit = std::min<int64_t>(N, std::max<int64_t>(N / 16, int64_t(c->num_sms) * 4 * 64));
   JoinCtl cached = cache_ctl ? *cache_ctl : plain;
   cached.row_limit = plain.row_limit;
-  auto sweep = [&](const JoinCtl* ctl, std::pair<int, int>* out) {
+  auto sweep = [&](const JoinCtl* ctl, bool far_only, int reps, JoinForm* out) {
     float best_ms = 1e30f;
-    for (int rep = 0; rep < kTuneReps; ++rep)
-      for (const auto& cf : cand) {
+    for (int rep = 0; rep < reps; ++rep)
+      for (const JoinForm& cf : cand) {
+        if (far_only && !cf.far) continue;
         cudaEventRecord(c->jev[0], c->stream);
         if (launch_join(c->codes.as<int8_t>(), c->join_sketch(), N, d, K, K * p.rerank_mult, ids[0], scs[0],
-                        ids[1], scs[1], order, scratch_counters, c->num_sms, c->stream, nullptr, ctl, cf.first,
-                        cf.second, c->sketch_words(d)) != cudaSuccess)
+                        ids[1], scs[1], order, scratch_counters, c->num_sms, c->stream, nullptr, ctl, cf.ctas,
+                        cf.cblock, c->sketch_words(d), cf.far) != cudaSuccess)
           return false;
         cudaEventRecord(c->jev[1], c->stream);
         cudaEventSynchronize(c->jev[1]);
@@ -376,14 +393,14 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
       }
     return true;
   };
-  if (!sweep(&plain, &best.early)) return best;
+  if (!sweep(&plain, far_early, kEarlyReps, &best.early)) return best;
   best.late = best.early;
   if (cache_ctl) {
     if (cudaMemsetAsync(cache_ctl->cache_cnt, 0, size_t(N) * 4, c->stream) != cudaSuccess ||
         launch_join(c->codes.as<int8_t>(), c->join_sketch(), N, d, K, K * p.rerank_mult, ids[0], scs[0],
                     ids[1], scs[1], order, scratch_counters, c->num_sms, c->stream, nullptr, &cached,
-                    best.early.first, best.early.second, c->sketch_words(d)) != cudaSuccess ||
-        !sweep(&cached, &best.late))
+                    best.early.ctas, best.early.cblock, c->sketch_words(d), best.early.far) != cudaSuccess ||
+        !sweep(&cached, false, kLateReps, &best.late))
       return best;
   }
   c->tuned[key] = best;
@@ -421,7 +438,7 @@ cudaError_t join_iterations(knng_ctx* c, const JoinPhase& ph, int from, int to,
     cudaError_t e;
     if ((e = launch_join(c->codes.as<int8_t>(), c->join_sketch(), ph.N, ph.d, K, K * p.rerank_mult, ph.ids[cur],
                          ph.scs[cur], ph.ids[nxt], ph.scs[nxt], ph.order, ph.ctl.counters, c->num_sms, c->stream,
-                         &ph.jt, &ci, cfg.first, cfg.second, c->sketch_words(ph.d))))
+                         &ph.jt, &ci, cfg.ctas, cfg.cblock, c->sketch_words(ph.d), cfg.far)))
       return (*step = "join launch", e);
     if ((e = launch_stop_check(ph.jt, ph.ctl, K, nxt, p.early_stop_rate, p.rate_diff_tol, loop, c->stream)))
       return (*step = "stop check", e);
@@ -626,8 +643,8 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
   if (skip_rows && (e = cudaMemsetAsync(c->rowflags.p, 1, size_t(N), str))) return cuda_fail(c, e, "row flag reset");
   // NN-Descent, captured once per launch key and replayed
   bool graph_used = false;
-  if ((e = join_prepare(K, K * p.rerank_mult, d, cfg.early.first, cfg.early.second)) ||
-      (e = join_prepare(K, K * p.rerank_mult, d, cfg.late.first, cfg.late.second)))
+  if ((e = join_prepare(K, K * p.rerank_mult, d, cfg.early.ctas, cfg.early.cblock, cfg.early.far)) ||
+      (e = join_prepare(K, K * p.rerank_mult, d, cfg.late.ctas, cfg.late.cblock, cfg.late.far)))
     return cuda_fail(c, e, (std::string("join variant: ") + join_variant_error()).c_str());
   const char* step = "";
   const JoinPhase ph{N, d, {ids[0], ids[1]}, {scs[0], scs[1]}, order, jt, ctl, cfg};
@@ -636,8 +653,9 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
                                         uintptr_t(c->jobs.p), uintptr_t(c->perm.p), uintptr_t(ctl.cache_ids),
                                         uintptr_t(c->rowflags.p),
                                         uintptr_t(N), uintptr_t(d),
-                                        uintptr_t(J), uintptr_t(o), uintptr_t(cfg.early.first), uintptr_t(cfg.early.second),
-                                        uintptr_t(cfg.late.first), uintptr_t(cfg.late.second),
+                                        uintptr_t(J), uintptr_t(o), uintptr_t(cfg.early.ctas), uintptr_t(cfg.early.cblock),
+                                        uintptr_t(cfg.late.ctas), uintptr_t(cfg.late.cblock),
+                                        uintptr_t(cfg.early.far), uintptr_t(cfg.late.far),
                                         uintptr_t(order != nullptr), uintptr_t(p.join_mode), uintptr_t(MI),
                                         uintptr_t(K), uintptr_t(p.rerank_mult)};
     if (!c->join_graph || c->join_graph_key != key) {
@@ -737,8 +755,8 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
   }
   S.forest_levels = levels;
   S.leaves = leaves;
-  S.join_ctas_per_sm = cfg.late.first;  // the configuration of the later iterations
-  S.join_cblock = cfg.late.second;
+  S.join_ctas_per_sm = cfg.late.ctas;  // the configuration of the later iterations
+  S.join_cblock = cfg.late.cblock;
   S.graph_used = graph_used ? 1 : 0;
   S.kernel_launches = launches() - launches0;
   S.total_s = std::chrono::duration<double>(clk::now() - t_start).count();
@@ -955,7 +973,7 @@ int knng_join_iter(knng_ctx* c, const int8_t* codes_dev, const uint64_t* sketch_
       return cuda_fail(c, e, "check word reset");
     if ((e = launch_join(codes_dev, sketch_dev, n, d, K, K * c->prm.rerank_mult, ids_in, scores_in, ids_out,
                          scores_out, nullptr, up, c->num_sms, c->stream, nullptr, kChecked ? &chk : nullptr, cps, cb,
-                         c->sketch_words(d))))
+                         c->sketch_words(d), !c->prm.join_ctas_per_sm && join_far(n, d))))
       return cuda_fail(c, e, "join");
     unsigned long long h = 0;
     unsigned check = 0;

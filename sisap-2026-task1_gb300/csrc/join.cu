@@ -55,8 +55,18 @@
 // sketch or 2 for the optional 128-hyperplane sketch (hyperplane.cu); the
 // score is 1024 - popcount over the W words either way.
 //
-// Stages per row (shared memory, K = 50, R = 400, d = 1024: ~53 KB); thread t
-// owns the occurrences j = t + 256r in every stage:
+// What bounds it: instruction issue (63 % busy) and the shared-memory pipe
+// (58 %) with four CTAs per SM and a barrier between stages, about 20,000 warp
+// instructions per computed row; the first two iterations, where most
+// candidates are new, the gathers of sketches and code rows.  Forms that only
+// shorten latencies (next row's two-hop ids fetched early, two table losers per
+// step, wider threshold scans) changed nothing or cost 1 to 4 %.
+// 100,000 x 1024: the phase takes 9.8 ms (probing tables: 19.2), an iteration
+// of 300,000 x 1024 rows of 64-dimensional data 22.7 ms (46.6).
+//
+// Stages per row (shared memory, K = 50, R = 400: 54 KB, FAR 48 KB); thread t
+// owns the occurrences j = 2p and 2p + 1 of the pairs p = t + 256r in every
+// stage:
 //   A  own list (loaded while the previous row was computed); the unchanged-
 //      row test; start copying the row's cache entries, code row and sketch
 //      into shared memory (cp.async)
@@ -71,8 +81,9 @@
 //      h_t from it
 //   E  selection: every occurrence with h > h_t plus the first
 //      R - count(h > h_t) occurrences with h == h_t in j order, ranked by
-//      ballot counts per (round, warp); the selected first occurrences that
-//      are neither starting-list members nor known to be rejected need a dot
+//      ballot counts per (round, warp), where a warp has a tie that could need
+//      a dot; the selected first occurrences that are neither starting-list
+//      members nor known to be rejected need one
 //   F  dp4a dots, a warp per four candidates (short rows: 8 lanes each); keep
 //      those above the starting pool[K-1].score, flag the others as rejected
 //   G  write the row's cache (this iteration's distinct ids, h and flags);
@@ -108,16 +119,25 @@ constexpr uint32_t kJBits = 12;              // occurrence index j < kMaxK * kMa
 constexpr uint32_t kJMask = (1u << kJBits) - 1u;
 static_assert(kMaxK * kMaxK <= (1 << kJBits), "occurrence index");
 constexpr uint32_t kTagTop = 0xffffeu;       // tags count down from here; 0xfffff marks a cleared slot
+static_assert(2 * kMaxPairs <= 16 && kMaxPairs * kThreads * 2 < int(0x8000), "an occurrence's bit and entry");
 constexpr int kTableB = 1024;                // second table (odd rounds): slots
 constexpr int kTableBShift = 22;
 constexpr uint32_t kXMask = 0x7ffu;          // info bits 0..10: Hamming distance
 constexpr uint32_t kKnown = 0x800u;          // info bit 11: distance taken from the row's candidate cache
 constexpr uint32_t kRej = 0x1000u;           // info bit 12: dot known to be <= the row's pool threshold
+constexpr uint32_t kPtr = 0x8000u;           // (FAR) entry bit 15: bits 0..14 are the id's first occurrence
 constexpr uint32_t kNone = 0xffffffffu;      // ids: no candidate (no id equals it: num_trees * n < 2^31)
 // The default parameters get a kernel of their own whose sizes and
 // shared-memory offsets are compile-time constants: read from the parameter
 // block they cost about 4,000 more instructions per row.
 constexpr int kDefK = 50, kDefR = 400;
+// FAR form of that kernel: 49 KB of shared memory per CTA instead of 55, which
+// leaves four CTAs 60 KB of L1 instead of 28.  Gathers in flight hold L1
+// lines, and with rows that come from beyond L2 there are many of them: at
+// 300,000 x 1024 (64-dimensional data) the first iteration reads the same
+// 113 GB of DRAM in 23.2 ms instead of 33.7.  It saves the space by keeping an
+// occurrence's info word and its pointer to the id's first occurrence in one
+// entry, and the survivors in the first table, at 2 % more instructions.
 
 // Shared-memory layout of one CTA (byte offsets).
 struct JoinLayout {
@@ -126,6 +146,8 @@ struct JoinLayout {
   int ta_slots, ta_shift;  // first table: slots and hash shift
   uint32_t kdiv;           // j / K = (j * kdiv) >> 20 for j < 4096
   uint32_t dummy;          // info index of occurrences without a candidate
+  uint32_t kp;             // words of a starting list
+  uint32_t survivors;      // most survivors of a row
   uint32_t o_code, o_sk, o_ids, o_rep, o_info, o_ta, o_tb, o_hist, o_x, o_pool, o_row, o_cell, o_member;
   uint32_t bytes;
 };
@@ -133,7 +155,7 @@ struct JoinLayout {
 __host__ __device__ constexpr uint32_t align16(uint32_t x) { return (x + 15u) & ~15u; }
 __host__ __device__ constexpr uint32_t umax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
-__host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool def) {
+__host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool def, bool far) {
   JoinLayout s{};
   s.KK = K * K;
   s.pairs = (s.KK + 1) / 2;
@@ -145,12 +167,15 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
     s.ta_slots <<= 1;
     --s.ta_shift;
   }
-  const uint32_t kk = uint32_t(2 * s.pairs), r = uint32_t(R);
+  const uint32_t kk = uint32_t(2 * s.pairs), r = uint32_t(R < s.KK ? R : s.KK);
+  const uint32_t rounds = uint32_t(def ? (s.pairs + kThreads - 1) / kThreads : kMaxPairs);
+  s.survivors = r;
+  s.kp = uint32_t(def ? K : kMaxK);
   // behind every occurrence index that a thread of the kernel forms
-  s.dummy = uint32_t(def ? (s.pairs + kThreads - 1) / kThreads : kMaxPairs) * kThreads * 2;
+  s.dummy = rounds * kThreads * 2;
   uint32_t o = 0;
   s.o_ids = o;   o += align16(4 * kk);
-  s.o_rep = o;   o += align16(umax(2 * kk, 14 * r));  // representatives, then the survivors' keys, ids and order
+  s.o_rep = o;   o += far ? 0 : align16(umax(2 * kk, 14 * r));  // representatives, then the survivors' keys, ids and order
   s.o_info = o;  o += 2 * s.dummy + 16;
   s.o_ta = o;    o += uint32_t(s.ta_slots) * 4;
   s.o_tb = o;    o += kTableB * 4;
@@ -158,15 +183,17 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
   // staged cached ids, then the warps' miss lists, then the rerank list, then
   // the ids of the row's next cache
   s.o_x = o;     o += align16(umax(umax(kCacheCap * 4, uint32_t((s.pairs + kThreads - 1) / kThreads) * kThreads * 4), 2 * r));
-  s.o_pool = o;  o += 2 * 2 * kMaxK * 4;  // starting lists of this row and of the previous one: ids, scores
+  s.o_pool = o;  o += align16(2 * 2 * s.kp * 4);  // starting lists of this row and of the previous one: ids, scores
   s.o_row = o;   o += 2 * 32;             // row counters, by row parity
-  s.o_cell = o;  o += align16(kMaxPairs * kWarps * 4);  // threshold ties per (round, warp)
-  s.o_member = o; o += kThreads * 4;      // per thread: its occurrences whose id is in the starting list
+  s.o_cell = o;  o += align16(rounds * kWarps * 4);  // threshold ties per (round, warp)
+  s.o_member = o; o += kThreads * 2;      // 16 bits per thread: its occurrences whose id is in the starting list
   s.o_sk = o;    o += 128;                // the widest sketch
   s.o_code = o;  o += align16(uint32_t(d));
   s.bytes = o;
   return s;
 }
+static_assert(join_layout(kDefK, kDefR, kMaxDim, true, true).bytes <= 49072, "four FAR CTAs in 196 KB");
+static_assert(join_layout(kDefK, kDefR, kMaxDim, true, true).ta_slots * 4 >= 14 * kDefR, "survivors in the first table");
 static_assert(kHBins * 4 >= kCacheCap * 2, "the histogram region stages the cached distances");
 
 // A row's counters (byte offsets from its set's start).
@@ -238,20 +265,39 @@ __device__ __forceinline__ void table_insert(uint32_t& id, uint32_t n, uint32_t 
 // Settle an occurrence j of `id` whose slot's winner w holds id `got`: a loser
 // enters the next round's table and sets its bit in `todo`; the winner itself
 // sets its bit in `first`.
-__device__ __forceinline__ void table_settle(uint32_t id, uint32_t got, uint32_t& w, uint32_t dummy, uint32_t j, uint32_t next_slot,
+template <bool FAR>
+__device__ __forceinline__ void table_settle(uint32_t id, uint32_t got, uint32_t& w, uint32_t dummy, uint32_t j, uint32_t a_info, uint32_t next_slot,
                                              uint32_t next_val, unsigned& todo, unsigned& first, unsigned bit) {
-  asm volatile(
-      "{\n.reg .pred p, q;\n"
-      "setp.ne.u32 q, %3, 0xffffffff;\n"
-      "selp.b32 %2, %2, %5, q;\n"
-      "setp.ne.and.u32 p, %4, %3, q;\n"
-      "@p red.shared.min.u32 [%7], %8;\n"
-      "@p or.b32 %0, %0, %9;\n"
-      "setp.eq.u32 q, %2, %6;\n"
-      "@q or.b32 %1, %1, %9;\n}"
-      : "+r"(todo), "+r"(first), "+r"(w)
-      : "r"(id), "r"(got), "r"(dummy), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit)
-      : "memory");
+  if (FAR) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n.reg .b32 t;\n"
+        "setp.ne.u32 q, %3, 0xffffffff;\n"
+        "selp.b32 %2, %2, %5, q;\n"
+        "setp.ne.and.u32 p, %4, %3, q;\n"
+        "@p red.shared.min.u32 [%7], %8;\n"
+        "@p or.b32 %0, %0, %9;\n"
+        "setp.eq.u32 q, %2, %6;\n"
+        "@q or.b32 %1, %1, %9;\n"
+        "or.pred p, p, q;\n"
+        "or.b32 t, %2, 0x8000;\n"
+        "@!p st.shared.u16 [%10], t;\n}"
+        : "+r"(todo), "+r"(first), "+r"(w)
+        : "r"(id), "r"(got), "r"(dummy), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit), "r"(a_info + 2 * j)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.u32 q, %3, 0xffffffff;\n"
+        "selp.b32 %2, %2, %5, q;\n"
+        "setp.ne.and.u32 p, %4, %3, q;\n"
+        "@p red.shared.min.u32 [%7], %8;\n"
+        "@p or.b32 %0, %0, %9;\n"
+        "setp.eq.u32 q, %2, %6;\n"
+        "@q or.b32 %1, %1, %9;\n}"
+        : "+r"(todo), "+r"(first), "+r"(w)
+        : "r"(id), "r"(got), "r"(dummy), "r"(j), "r"(next_slot), "r"(next_val), "r"(bit)
+        : "memory");
+  }
 }
 // Look a cached id up in round 0: `e` is its slot, `base` the round's tag.  A
 // slot of an older round: absent.  Else the winner's id decides: equal, and the
@@ -318,6 +364,18 @@ __device__ __forceinline__ void cache_push(unsigned m, unsigned bit, uint32_t& a
       : "+r"(at_id), "+r"(at_info)
       : "r"(m), "r"(bit), "r"(end), "r"(id), "r"(info)
       : "memory");
+}
+// (FAR) The info word behind an entry: its own, or that of the first occurrence it points to.
+__device__ __forceinline__ uint32_t info_of(uint32_t e, uint32_t a_info) {
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b32 a;\n"
+      "setp.ge.u32 p, %0, 0x8000;\n"
+      "mad.lo.u32 a, %0, 2, %1;\n"
+      "@p ld.shared.u16 %0, [a + -65536];\n}"
+      : "+r"(e)
+      : "r"(a_info)
+      : "memory");
+  return e;
 }
 __device__ __forceinline__ void red_or(uint32_t a, uint32_t v) {
   asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -481,7 +539,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // CB: sketches in flight per 8-lane group (Hamming stage); MINB: resident CTAs
 // per SM the register budget allows; DEF: the default K and R (and 8-byte
 // aligned input lists), else any.
-template <int CB, int MINB, bool DEF>
+template <int CB, int MINB, bool DEF, bool FAR>
 __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     const int8_t* __restrict__ codes, const uint64_t* __restrict__ sketch, int64_t n64, int d, int K_, int R_, int W,
     const int32_t* ids_in, const int32_t* scores_in, int32_t* ids_out, int32_t* scores_out,
@@ -495,7 +553,8 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     counters += 8 * it;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl.times[2 * it] = global_ns();
   }
-  constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim, true);
+  static_assert(DEF || !FAR, "FAR is a form of the default kernel");
+  constexpr JoinLayout LD = join_layout(kDefK, kDefR, kMaxDim, true, FAR);
 #define KNNG_L(f) (DEF ? LD.f : LA.f)
   constexpr int NP = DEF ? (LD.pairs + kThreads - 1) / kThreads : kMaxPairs;  // pairs per thread
   const int K = DEF ? kDefK : K_, R = DEF ? kDefR : R_;
@@ -514,8 +573,11 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
   const uint32_t a_ta = sb + KNNG_L(o_ta), a_tb = sb + KNNG_L(o_tb), a_hist = sb + KNNG_L(o_hist);
   const uint32_t a_x = sb + KNNG_L(o_x), a_cell = sb + KNNG_L(o_cell), a_code = sb + KNNG_L(o_code);
   const uint32_t a_member = sb + KNNG_L(o_member);
-  // survivors: 64-bit keys {dot, visit key}, then ids, then (sequential insertion) their visit order
-  const uint32_t a_sid = a_rep + 8u * uint32_t(R), a_sorder = a_rep + 12u * uint32_t(R);
+  // survivors: 64-bit keys {dot, visit key}, then ids, then (sequential
+  // insertion) their visit order; with FAR over the first table, which stage F
+  // no longer reads
+  const uint32_t a_key = FAR ? a_ta : a_rep;
+  const uint32_t a_sid = a_key + 8u * KNNG_L(survivors), a_sorder = a_key + 12u * KNNG_L(survivors);
   // per-CTA statistics, kept by thread 0 in shared memory (no registers held
   // across the row loop): updates, sketches scored, rows reranked, distinct
   // candidates, rows skipped
@@ -539,7 +601,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     for (int t = tid; t < kTableB / 4; t += kThreads) sts128(a_tb + 16 * t, e);
   };
   clear_tables();
-  sts32(a_member + 4 * tid, 0);
+  sts16(a_member + 2 * tid, 0);
   uint32_t tag = kTagTop;           // block-uniform
   uint32_t par = 0;                 // parity of the computed rows
 
@@ -580,9 +642,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
   auto fetch_list = [&](uint32_t to) {  // list and cache count of row nx_i
     if (nx_i >= 0 && KNNG_GUARD(ctl.check_err, nx_i < int(n))) {
       if (tid < K) {
-        const uint32_t dst = sb + KNNG_L(o_pool) + to * (2u * kMaxK * 4u) + 4u * uint32_t(tid);
+        const uint32_t dst = sb + KNNG_L(o_pool) + to * (8u * KNNG_L(kp)) + 4u * uint32_t(tid);
         cp_async4(dst, ids_in + int64_t(nx_i) * K + tid);
-        cp_async4(dst + kMaxK * 4u, scores_in + int64_t(nx_i) * K + tid);
+        cp_async4(dst + 4u * KNNG_L(kp), scores_in + int64_t(nx_i) * K + tid);
       }
       if (cached) nx_cc = ctl.cache_cnt[nx_i];
     }
@@ -599,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     if (tid <= K && nx_i >= 0 && (!kChecked || nx_i < int(n))) {
       nx_flag = 1;
       if (ctl.chg_in) {
-        const uint32_t at = tid < K ? lds32(sb + KNNG_L(o_pool) + to * (2u * kMaxK * 4u) + 4u * uint32_t(tid)) : uint32_t(nx_i);
+        const uint32_t at = tid < K ? lds32(sb + KNNG_L(o_pool) + to * (8u * KNNG_L(kp)) + 4u * uint32_t(tid)) : uint32_t(nx_i);
         if (at < n) nx_flag = int(ctl.chg_in[at]);
       }
       if (ctl.job_done) {
@@ -626,8 +688,8 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       continue;
     }
     // ---- A
-    const uint32_t a_pool = sb + KNNG_L(o_pool) + slot * (2u * kMaxK * 4u);  // ids; scores kMaxK words on
-    const uint32_t a_psc = a_pool + kMaxK * 4u;
+    const uint32_t a_pool = sb + KNNG_L(o_pool) + slot * (8u * KNNG_L(kp));  // ids, then scores
+    const uint32_t a_psc = a_pool + 4u * KNNG_L(kp);
     const uint32_t a_row = sb + KNNG_L(o_row) + 32u * par;
     const bool work = __syncthreads_or(moved) != 0;  // block-uniform
     finish_row();
@@ -750,11 +812,11 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const uint32_t id = v[2 * r + e];
-          table_settle(id, lds32(a_ids + 4 * w[2 * r + e]), w[2 * r + e], KNNG_L(dummy), uint32_t(2 * p + e),
-                       a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e), todo,
-                       fm, 1u << (2 * r + e));
+          table_settle<FAR>(id, lds32(a_ids + 4 * w[2 * r + e]), w[2 * r + e], KNNG_L(dummy), uint32_t(2 * p + e), a_info,
+                            a_tb + slot_of(id, 1u, kTableBShift), tagj - (1u << kJBits) + uint32_t(2 * kThreads * r + e), todo,
+                            fm, 1u << (2 * r + e));
         }
-        if (p < KNNG_L(pairs)) sts32(a_rep + 4 * p, w[2 * r] | (w[2 * r + 1] << 16));
+        if (!FAR && p < KNNG_L(pairs)) sts32(a_rep + 4 * p, w[2 * r] | (w[2 * r + 1] << 16));
       }
     }
 #pragma unroll 1
@@ -791,9 +853,10 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         const uint32_t id = lds32(a_ids + 4 * j);
         const uint32_t w = lds32(t_cur + slot_of(id, round, sh_cur)) & kJMask;
         if (lds32(a_ids + 4 * w) == id) {
-          sts16(a_rep + 2 * j, w);
+          if (!FAR) sts16(a_rep + 2 * j, w);
           todo ^= 1u << b;
           if (w == j) fm |= 1u << b;
+          else if (FAR) sts16(a_info + 2 * j, w | kPtr);
         } else {
           red_min(t_nxt + slot_of(id, round + 1u, sh_nxt), ((tc - 1u) << kJBits) + j);
         }
@@ -827,9 +890,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     // ---- C  Hamming once per distinct id without a cached distance: each warp
     //         lists its own first occurrences that are misses and scores them
     //         (groups of 8 lanes, CB candidates in flight per group)
-    if (find_rep >= 0) {  // occurrence 2 (t + 256 r) + e: bit 2r + e of thread t's word
-      const uint32_t p = uint32_t(find_rep) >> 1;
-      red_or(a_member + 4 * (p % kThreads), 1u << (2 * (p / kThreads) + (uint32_t(find_rep) & 1u)));
+    if (find_rep >= 0) {  // occurrence 2 (t + 256 r) + e: bit 2r + e of thread t's half word
+      const uint32_t p = uint32_t(find_rep) >> 1, t = p % kThreads;
+      red_or(a_member + 4 * (t >> 1), 1u << (16 * (t & 1u) + 2 * (p / kThreads) + (uint32_t(find_rep) & 1u)));
     }
     for (int t = tid; t < kHBins / 4; t += kThreads) sts128(a_hist + 16 * t, make_uint4(0, 0, 0, 0));
     int first_at;  // this thread's place among the row's distinct ids (stage G)
@@ -931,8 +994,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       const int p = tid + kThreads * r;
       hv[r] = kNoDist | (kNoDist << 16);
       if (p < KNNG_L(pairs)) {
-        const uint32_t w = lds32(a_rep + 4 * p);
-        const uint32_t f0 = lds16(a_info + 2 * (w & 0xffffu)), f1 = lds16(a_info + 2 * (w >> 16));
+        const uint32_t w = lds32((FAR ? a_info : a_rep) + 4 * p);
+        const uint32_t f0 = FAR ? info_of(w & 0xffffu, a_info) : lds16(a_info + 2 * (w & 0xffffu));
+        const uint32_t f1 = FAR ? info_of(w >> 16, a_info) : lds16(a_info + 2 * (w >> 16));
         hv[r] = f0 | (f1 << 16);
         red_add(a_hist + 4 * (f0 & kXMask), 1u);
         red_add(a_hist + 4 * (f1 & kXMask), 1u);
@@ -986,8 +1050,8 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       mark_near(hv[r] & (kXMask | kRej), hv[r] & kXMask, xt, wm, eqm, open, 1u << (2 * r));
       mark_near(hv[r] & ((kXMask | kRej) << 16), hv[r] & (kXMask << 16), xt << 16, wm, eqm, open, 2u << (2 * r));
     }
-    const unsigned want = fm & ~lds32(a_member + 4 * tid);
-    sts32(a_member + 4 * tid, 0);
+    const unsigned want = fm & ~lds16(a_member + 2 * tid);
+    sts16(a_member + 2 * tid, 0);
     wm &= want;
     open &= want;
     if (cut) {
@@ -1036,7 +1100,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     __syncthreads();
     // ---- F  dots
     {
-      const DotSink sink{a_row, a_x, a_ids, a_info, a_psc + 4 * (K - 1), a_rep, a_sid, cached};
+      const DotSink sink{a_row, a_x, a_ids, a_info, a_psc + 4 * (K - 1), a_key, a_sid, cached};
       if (d > 512) dots_wide<2>(codes, d, uint32_t(i), a_code, tid, sink);  // uniform
       else if (d > 256) dots_wide<1>(codes, d, uint32_t(i), a_code, tid, sink);
       else if (d > 128) dots_narrow<2>(codes, a_code, tid, sink);
@@ -1093,7 +1157,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
           id = lds32(a_pool + 4 * u);
           rank = u;
         } else {
-          const uint2 k2 = lds64(a_rep + 8 * (u - K));
+          const uint2 k2 = lds64(a_key + 8 * (u - K));
           me = (uint64_t(k2.y) << 32) | k2.x;
           id = lds32(a_sid + 4 * (u - K));
           const int32_t dot = int32_t(k2.y ^ 0x80000000u);
@@ -1108,12 +1172,12 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         int q = 0;
 #pragma unroll 2
         for (; q + 1 < P; q += 2) {
-          const uint4 o = lds128(a_rep + 8 * q);
+          const uint4 o = lds128(a_key + 8 * q);
           rank += ((uint64_t(o.y) << 32) | o.x) > me ? 1 : 0;
           rank += ((uint64_t(o.w) << 32) | o.z) > me ? 1 : 0;
         }
         if (q < P) {
-          const uint2 o = lds64(a_rep + 8 * q);
+          const uint2 o = lds64(a_key + 8 * q);
           rank += ((uint64_t(o.y) << 32) | o.x) > me ? 1 : 0;
         }
         if (rank < K) {
@@ -1132,9 +1196,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
       // loop in warp 0 with the pool held two entries per lane
 #pragma unroll 1
       for (int p = tid; p < P; p += kThreads) {
-        const uint32_t kp = lds32(a_rep + 8 * p);
+        const uint32_t kp = lds32(a_key + 8 * p);
         int rank = 0;
-        for (int q = 0; q < P; ++q) rank += lds32(a_rep + 8 * q) > kp ? 1 : 0;
+        for (int q = 0; q < P; ++q) rank += lds32(a_key + 8 * q) > kp ? 1 : 0;
         sts16(a_sorder + 2 * rank, uint32_t(p));
       }
       __syncthreads();
@@ -1146,7 +1210,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
 #pragma unroll 1
         for (int rr = 0; rr < P; ++rr) {
           const uint32_t p = lds16(a_sorder + 2 * rr);
-          const int32_t id = int32_t(lds32(a_sid + 4 * p)), dot = int32_t(lds32(a_rep + 8 * p + 4) ^ 0x80000000u);
+          const int32_t id = int32_t(lds32(a_sid + 4 * p)), dot = int32_t(lds32(a_key + 8 * p + 4) ^ 0x80000000u);
           if (__any_sync(full, idA == id || idB == id)) continue;
           const int32_t last = (K - 1) < 32 ? __shfl_sync(full, scA, K - 1) : __shfl_sync(full, scB, K - 33);
           if (!(dot > last)) continue;
@@ -1183,8 +1247,16 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
         if (lane == 0) sts32(a_row + kRowChanged, uint32_t(changed));
       }
     }
+    if (cached || (FAR && P > 0)) __syncthreads();  // block-uniform
+    if (FAR) {  // the slots that held survivors are empty again before the next row's first barrier
+#pragma unroll 1
+      for (int p = tid; p < P; p += kThreads) {
+        sts64(a_key + 8 * p, ~0u, ~0u);
+        sts32(a_sid + 4 * p, ~0u);
+        if (serial_insert) sts16(a_sorder + 2 * p, 0xffffu);
+      }
+    }
     if (cached) {
-      __syncthreads();
       const int nc = min(int(lds32(a_row + kRowNu)), ctl.cache_cap);
       uint4* cid = reinterpret_cast<uint4*>(ctl.cache_ids + int64_t(i) * ctl.cache_cap);
       uint4* chr = reinterpret_cast<uint4*>(ctl.cache_hr + int64_t(i) * ctl.cache_cap);
@@ -1264,19 +1336,30 @@ using JoinKernel = void (*)(const int8_t*, const uint64_t*, int64_t, int, int, i
 
 // ctas_per_sm 3: up to 80 registers per thread, 3 resident CTAs; otherwise 64
 // registers, 4 resident CTAs.
-template <bool DEF>
+template <bool DEF, bool FAR>
 JoinKernel pick_variant(int ctas_per_sm, int cblock) {
   if (ctas_per_sm == 3)
-    return cblock == 2 ? join_kernel<2, 3, DEF> : cblock == 8 ? join_kernel<8, 3, DEF> : join_kernel<4, 3, DEF>;
-  return cblock == 2 ? join_kernel<2, 4, DEF> : cblock == 8 ? join_kernel<8, 4, DEF> : join_kernel<4, 4, DEF>;
+    return cblock == 2 ? join_kernel<2, 3, DEF, FAR> : cblock == 8 ? join_kernel<8, 3, DEF, FAR> : join_kernel<4, 3, DEF, FAR>;
+  return cblock == 2 ? join_kernel<2, 4, DEF, FAR> : cblock == 8 ? join_kernel<8, 4, DEF, FAR> : join_kernel<4, 4, DEF, FAR>;
 }
 // The kernel and shared-memory layout of a launch: the default K and R have
 // their own kernel, which reads the lists 8 bytes at a time (`aligned`).
-JoinKernel variant(int K, int R, int d, bool aligned, int ctas_per_sm, int cblock, JoinLayout* L) {
+JoinKernel variant(int K, int R, int d, bool aligned, int ctas_per_sm, int cblock, bool far, JoinLayout* L) {
   const bool def = K == kDefK && R == kDefR && aligned;
-  *L = join_layout(K, R, def ? kMaxDim : d, def);
-  return def ? pick_variant<true>(ctas_per_sm, cblock) : pick_variant<false>(ctas_per_sm, cblock);
+  far = far && def;
+  *L = join_layout(K, R, def ? kMaxDim : d, def, far);
+  if (far) return pick_variant<true, true>(ctas_per_sm, cblock);
+  return def ? pick_variant<true, false>(ctas_per_sm, cblock) : pick_variant<false, false>(ctas_per_sm, cblock);
 }
+
+bool join_has_far(int K, int R) { return K == kDefK && R == kDefR; }
+
+// While most candidates are new, the FAR form is the faster one from about
+// where the codes outgrow L2.  First iteration with four CTAs, without / with
+// it: 100,000 x 1024 3.82 / 3.78 ms, 150,000 x 1024 6.24 / 6.04, 300,000 x 1024
+// 14.6 / 13.4, 600,000 x 1024 33.7 / 29.4, 300,000 x 384 11.87 / 11.98,
+// 600,000 x 384 26.6 / 26.5.
+bool join_far(int64_t n, int d) { return n * d >= int64_t(120) << 20; }
 
 cudaError_t max_ctas(JoinKernel kern, int ctas_per_sm, int cblock, uint32_t smem, int* per_sm_out) {
   std::lock_guard<std::mutex> lk(g_variant_mu);
@@ -1315,17 +1398,18 @@ const char* join_variant_error() { return g_variant_err; }
 
 cudaError_t join_prepare_all(int K, int R, int d) {
   for (int c : {3, 4})
-    for (int b : {2, 4, 8}) {
-      const cudaError_t e = join_prepare(K, R, d, c, b);
-      if (e != cudaSuccess) return e;
-    }
+    for (int b : {2, 4, 8})
+      for (bool far : {false, true}) {
+        const cudaError_t e = join_prepare(K, R, d, c, b, far);
+        if (e != cudaSuccess) return e;
+      }
   return cudaSuccess;
 }
 
-cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock) {
+cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock, bool far) {
   JoinLayout L;
   int per_sm = 0;
-  const JoinKernel kern = variant(K, R, d, true, ctas_per_sm, cblock, &L);
+  const JoinKernel kern = variant(K, R, d, true, ctas_per_sm, cblock, far, &L);
   return max_ctas(kern, ctas_per_sm, cblock, L.bytes, &per_sm);
 }
 
@@ -1341,9 +1425,9 @@ cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int
 cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, int d, int K, int R,
                         const int32_t* ids_in, const int32_t* scores_in, int32_t* ids_out, int32_t* scores_out,
                         const int32_t* row_order, unsigned long long* counters, int num_sms, cudaStream_t s,
-                        const JobTable* jt, const JoinCtl* ctl, int ctas_per_sm, int cblock, int sk_words) {
+                        const JobTable* jt, const JoinCtl* ctl, int ctas_per_sm, int cblock, int sk_words, bool far) {
   JoinLayout L;
-  const JoinKernel kern = variant(K, R, d, (reinterpret_cast<uintptr_t>(ids_in) & 7) == 0, ctas_per_sm, cblock, &L);
+  const JoinKernel kern = variant(K, R, d, (reinterpret_cast<uintptr_t>(ids_in) & 7) == 0, ctas_per_sm, cblock, far, &L);
   int per_sm = 1;
   KNNG_CUDA_TRY(max_ctas(kern, ctas_per_sm, cblock, L.bytes, &per_sm));
   const int64_t blocks = std::min<int64_t>(n, int64_t(num_sms) * per_sm);

@@ -282,11 +282,14 @@ cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, 
                         const int32_t* ids_in, const int32_t* scores_in, int32_t* ids_out,
                         int32_t* scores_out, const int32_t* row_order, unsigned long long* counters,
                         int num_sms, cudaStream_t s, const JobTable* jt = nullptr,
-                        const JoinCtl* ctl = nullptr, int ctas_per_sm = 0, int cblock = 4, int sk_words = 0);
+                        const JoinCtl* ctl = nullptr, int ctas_per_sm = 0, int cblock = 4, int sk_words = 0,
+                        bool far = false);
 // sk_words: 64-bit sketch words per row (0: d / 64, the sign sketch; 2: hyperplane sketch)
 // ctas_per_sm: 4 (64 registers per thread) or 3 (up to 85, no spills);
 // cblock: sketch candidates in flight per 8-lane group in the Hamming stage
-// (2, 4 or 8).  Both are chosen by the autotuner.
+// (2, 4 or 8); far: less shared memory per CTA and more L1, for rows that come
+// from beyond L2 (default K and R only, else ignored).  All three are chosen by
+// the autotuner; join_far says where far wins while candidates are new.
 // counters[0] += updates, counters[1] += sketches scored (distinct candidates
 // without a cached score), counters[2] += reranked rows, counters[3] +=
 // distinct candidates.
@@ -298,7 +301,9 @@ cudaError_t launch_join(const int8_t* codes, const uint64_t* sketch, int64_t n, 
 cudaError_t launch_stop_check(const JobTable& jt, const JoinCtl& ctl, int K, int out_buf, float stop_rate,
                               float diff_tol, const cudaGraphConditionalHandle* loop, cudaStream_t s);
 // Resolve a join variant's launch attributes before any stream capture.
-cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock);
+bool join_has_far(int K, int R);
+bool join_far(int64_t n, int d);
+cudaError_t join_prepare(int K, int R, int d, int ctas_per_sm, int cblock, bool far);
 cudaError_t join_prepare_all(int K, int R, int d);  // every variant the autotuner may pick
 const char* join_variant_error();                    // detail of the last failed resolution
 
