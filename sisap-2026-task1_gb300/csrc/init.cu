@@ -7,13 +7,15 @@
 // with random ids of score INT32_MIN.
 //
 // Here the dots come from one Gram block per leaf (K3: every member pair of a
-// <= 64-member leaf, read once from HBM into shared memory), and a warp per
-// row merges its T leaf rows into a sorted top-K list held two entries per
-// lane (K4), one batched merge per 32 candidates (merge_batch).  The merge keeps the K best distinct (score desc, id asc) keys,
-// which is the reference's pool order among equal scores (its pool is sorted
-// by id before the unstable partial_sort; ties are unspecified there and fixed
-// here).  Rows with fewer than K distinct candidates take the reference's
-// random-fill path exactly, one thread per row (tiny inputs only).
+// <= 64-member leaf, each code row read once; gram_mma.cu, gram_tc.cu, or the
+// dp4a form below), and a warp per row merges its T leaf rows into a sorted
+// top-K list held two entries per lane (K4), 32 candidates above the list's
+// last key at a time (merge_batch).  The merge keeps the K best distinct
+// (score desc, id asc) keys, which is the reference's pool order among equal
+// scores (its pool is sorted by id before the unstable partial_sort; ties are
+// unspecified there and fixed here).  Rows with fewer than K distinct
+// candidates take the reference's random-fill path exactly, one thread per row
+// (tiny inputs only).
 #include "knng_internal.cuh"
 
 #include <algorithm>
@@ -154,58 +156,65 @@ __device__ __forceinline__ uint64_t list_insert(uint64_t& kA, uint64_t& kB, uint
   return (K - 1) < 32 ? __shfl_sync(full, kA, K - 1) : __shfl_sync(full, kB, K - 33);
 }
 
-// Merge one leaf half's candidate keys (one per lane, 0 = none) into the
-// descending list kA/kB (positions lane and 32 + lane, length K; 0 = empty):
-// afterwards it holds the K best distinct keys of both.  One pass for all the
-// candidates above the threshold instead of one insertion each: the list goes
-// to the warp's shared-memory row; such a candidate finds its rank in the list
-// by binary search (an equal key is listed already) and its rank among the
-// other candidates by counting; every list entry moves down by the number of
-// candidates above it.  The ranks are a permutation of the merged order, so
-// each entry and candidate is written once, and those at rank >= K drop out.
-// Returns the new threshold (the K-th key, 0 while the list is not full).
+__device__ __forceinline__ uint64_t max64(uint64_t a, uint64_t b) { return a > b ? a : b; }
+__device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a > b ? b : a; }
+
+// Merge up to 32 candidate keys (one per lane, 0 = none, repeats allowed) into
+// the descending list kA/kB (positions lane and 32 + lane, length K; 0 = empty;
+// sl holds the same list): afterwards it holds the K best distinct keys of
+// both.  Repeats among the candidates and keys listed already (binary search
+// in sl) drop out; the rest are sorted across the warp, and the larger of list
+// and reversed candidates at every place is the best 64 of both in bitonic
+// order, which six exchange steps sort.  Returns the new threshold (the K-th
+// key, 0 while the list is not full).
+// Candidates wait in shared memory until 32 of them are above the threshold
+// (init_merge): a leaf half gives 6 on average, and a merge costs about 300
+// instructions for 1 or 32.  Bound by instructions; with a merge per leaf half
+// and ranks by counting the initial graph took 4.17 ms at 300k x 1024 and
+// 14.9 at 1M, now 3.54 and 13.3 (waiting alone, ranks by counting: 4.07, 15.0).
 __device__ __forceinline__ uint64_t merge_batch(uint64_t& kA, uint64_t& kB, uint64_t key, uint64_t thr, int K,
                                                 int lane, uint64_t* sl) {
   const unsigned full = 0xffffffffu;
-  bool want = key > thr;
-  if (!__any_sync(full, want)) return thr;
-  sl[lane] = kA;
-  sl[32 + lane] = kB;
-  __syncwarp();
-  int lo = 0;
+  // the first lane of an id: equal ids have equal keys, as a pair's dot is the
+  // same in every tree
+  const bool lead = __ffs(__match_any_sync(full, uint32_t(key))) - 1 == lane;
+  bool want = key > thr && lead;
   if (want) {
-    int hi = K;  // first list position whose key is <= key
+    int lo = 0, hi = K;  // first list position whose key is <= key
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       if (sl[mid] > key) lo = mid + 1;
       else hi = mid;
     }
-    if (lo < K && sl[lo] == key) want = false;
+    want = !(lo < K && sl[lo] == key);
   }
-  // the accepted candidates side by side (a 0 behind an odd count), two per
-  // load: one find-first and two shuffles per candidate, as before, cost 12 %
-  // of the kernel (1M rows, 16 trees: 9.0 -> 7.9 ms)
-  const unsigned acc = __ballot_sync(full, want);
-  const int na = __popc(acc);
-  uint64_t* cand = sl + kMaxK;
-  if (want) cand[__popc(acc & ((1u << lane) - 1u))] = key;
-  if (lane == 0 && na < 32) cand[na] = 0;
-  __syncwarp();
-  int above = 0, cA = 0, cB = 0;
-#pragma unroll 2
-  for (int q = 0; q < na; q += 2) {
-    const ulonglong2 ck = *reinterpret_cast<const ulonglong2*>(cand + q);
-    above += (ck.x > key ? 1 : 0) + (ck.y > key ? 1 : 0);
-    cA += (ck.x > kA ? 1 : 0) + (ck.y > kA ? 1 : 0);
-    cB += (ck.x > kB ? 1 : 0) + (ck.y > kB ? 1 : 0);
+  if (!__any_sync(full, want)) return thr;
+  uint64_t c = want ? key : 0;
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1)  // ascending
+#pragma unroll
+    for (int o = k >> 1; o > 0; o >>= 1) {
+      const uint64_t other = __shfl_xor_sync(full, c, o);
+      const bool keep_min = ((lane & k) == 0) == ((lane & o) == 0);
+      c = (c > other) == keep_min ? other : c;
+    }
+  kB = max64(kB, c);
+  const uint64_t hi = max64(kA, kB);
+  kB = min64(kA, kB);
+  kA = hi;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) == 0;  // keeps the larger
+    const uint64_t a = __shfl_xor_sync(full, kA, o), b = __shfl_xor_sync(full, kB, o);
+    kA = (kA > a) == up ? kA : a;
+    kB = (kB > b) == up ? kB : b;
   }
-  if (lane < K && lane + cA < K) sl[lane + cA] = kA;
-  if (32 + lane < K && 32 + lane + cB < K) sl[32 + lane + cB] = kB;
-  if (want && lo + above < K) sl[lo + above] = key;
+  if (lane >= K) kA = 0;
+  if (32 + lane >= K) kB = 0;
   __syncwarp();
-  kA = lane < K ? sl[lane] : 0;
-  kB = 32 + lane < K ? sl[32 + lane] : 0;
-  __syncwarp();  // the row is rewritten by the next merge
+  sl[lane] = kA;
+  sl[32 + lane] = kB;
+  __syncwarp();
   return (K - 1) < 32 ? __shfl_sync(full, kA, K - 1) : __shfl_sync(full, kB, K - 33);
 }
 
@@ -225,7 +234,9 @@ __global__ void __launch_bounds__(256) init_merge(int64_t n, int t0, int t1, int
                                                   int64_t gram_rows, unsigned* err) {
   (void)gram_rows;
   (void)err;
-  __shared__ __align__(16) uint64_t s_list[8][kMaxK + 32];  // one list row and 32 candidates per warp (merge_batch)
+  __shared__ uint64_t s_list[8][kMaxK + 64];  // per warp: its list, then the waiting candidates
+  uint64_t* const sl = s_list[threadIdx.x >> 5];
+  uint64_t* const wait = sl + kMaxK;
   const int lane = threadIdx.x & 31;
   const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
   for (int64_t i = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
@@ -241,6 +252,11 @@ __global__ void __launch_bounds__(256) init_merge(int64_t n, int t0, int t1, int
       }
       thr = (K - 1) < 32 ? __shfl_sync(0xffffffffu, kA, K - 1) : __shfl_sync(0xffffffffu, kB, K - 33);
     }
+    __syncwarp();
+    sl[lane] = kA;
+    sl[32 + lane] = kB;
+    __syncwarp();
+    int nw = 0;  // waiting candidates, fewer than 32 between halves
     for (int t = t0; t < t1; ++t) {
       const int64_t p = pos[int64_t(t) * n + i];
       // (bounds-checked build) the position lies in tree t, its leaf in the
@@ -253,12 +269,25 @@ __global__ void __launch_bounds__(256) init_merge(int64_t n, int t0, int t1, int
       const int32_t* grow = gram + (p - gram_pos0) * int64_t(kMaxLeaf);
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
+        if (32 * half >= m) break;  // warp-uniform
         const int j = lane + 32 * half;
         uint64_t key = 0;
         if (j < m && j != self) key = make_key(grow[j], perm[s + j]);
-        thr = merge_batch(kA, kB, key, thr, K, lane, s_list[threadIdx.x >> 5]);
+        const unsigned above = __ballot_sync(0xffffffffu, key > thr);
+        if (key > thr) wait[nw + __popc(above & ((1u << lane) - 1u))] = key;
+        nw += __popc(above);
+        if (nw >= 32) {
+          __syncwarp();
+          const uint64_t k0 = wait[lane], k1 = wait[32 + lane];  // k1: the first nw - 32 count
+          __syncwarp();
+          nw -= 32;
+          thr = merge_batch(kA, kB, k0, thr, K, lane, sl);
+          if (lane < nw) wait[lane] = k1;
+        }
       }
     }
+    __syncwarp();
+    thr = merge_batch(kA, kB, lane < nw ? wait[lane] : 0, thr, K, lane, sl);
     const int real = __popc(__ballot_sync(0xffffffffu, kA != 0)) + __popc(__ballot_sync(0xffffffffu, kB != 0));
     int32_t* gi = ids + i * K;
     int32_t* gs = scores + i * K;
