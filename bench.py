@@ -49,8 +49,8 @@ METRIC = "vectors/s (kNN-graph build, recall@15-checked)"
 GRAM = {"dp4a": 0, "tc": 1}
 # DRAM read + write bytes per row of one working NN-Descent launch: the mean
 # over the working join launches of one 300k x 1024 build (3k centres), from
-# the one-pass ncu capture summarised in profiles/join_kernel_dram_300k.md.
-JOIN_DRAM_BYTES_PER_ROW_300K = 22251.0
+# the ncu capture summarised in profiles/join_kernel_dram_300k.md.
+JOIN_DRAM_BYTES_PER_ROW_300K = 23341.0
 JOIN_TRAFFIC_SOURCE = ("profiles/join_kernel_dram_300k.md: mean DRAM bytes per row of a 300k build's working "
                        "join launches (ncu), times this workload's rows")
 
@@ -660,7 +660,7 @@ def run_gpu(args):
             "vs_baseline": None, "dtype": "int8/int32", "data": "synthetic (seeded Gaussian mixture, Zipf 1.1)",
             "config": workload_config(args.config, ws, prm),
             "implementation": {"join": "jacobi" if prm.join_mode == 0 else "inplace",
-                               "leaf_gram": "tcgen05 f16" if prm.gram_mode == 1 else "dp4a",
+                               "leaf_gram": "f16 tensor cores" if prm.gram_mode == 1 else "dp4a",
                                "forest": "three levels per pass" if prm.forest_fuse else "one level per pass",
                                "candidate_cache": bool(prm.join_cache),
                                "join_tuned": {"ctas_per_sm": last.join_ctas_per_sm, "cblock": last.join_cblock,
@@ -701,7 +701,7 @@ def main():
     ap.add_argument("--impl", default="gpu", choices=["gpu", "reference"])
     ap.add_argument("--config", default="full", choices=sorted(CONFIGS) + ["batched", "serving"])
     ap.add_argument("--gram", default="tc", choices=["tc", "dp4a"],
-                    help="leaf Gram: tcgen05 f16 tensor cores or dp4a")
+                    help="leaf Gram: f16 tensor cores or dp4a")
     ap.add_argument("--join-cache", type=int, default=1, choices=[0, 1],
                     help="per-row candidate cache in the NN-Descent join (identical results; 1 = default)")
     ap.add_argument("--forest-fuse", type=int, default=1, choices=[0, 1],

@@ -68,7 +68,8 @@ typedef struct knng_params {
   int device;            /* CUDA device ordinal */
   int autotune;          /* 1: time the join configurations once per (d, size) */
   int use_graph;         /* 1: replay the NN-Descent phase as a CUDA graph */
-  int gram_mode;         /* leaf Gram: KNNG_GRAM_DP4A or KNNG_GRAM_TCGEN05 (f16 tensor cores) */
+  int gram_mode;         /* leaf Gram: KNNG_GRAM_DP4A or KNNG_GRAM_TCGEN05 (f16 tensor cores: a
+                            warp per leaf from registers; tcgen05 where wait_limit is set) */
   int init_mode;         /* KNNG_INIT_FOREST (src/main.cpp); KNNG_INIT_RANDOM, the archived
                             variant archive/nndescent_optimized.cpp:97-118 (needs n > k_build);
                             KNNG_INIT_BLOCK, the archived block-partitioned hybrid
@@ -84,9 +85,10 @@ typedef struct knng_params {
                             (2, nndescent_hybrid.cpp:22); drawn with xorshift32 from seed + row */
   int wait_limit;        /* polls before a bounded device wait gives up with KNNG_E_TIMEOUT:
                             0 = the default (2^26); a negative value makes those waits give up
-                            at once (only used to test the timeout path).  The tensor-core leaf
-                            Gram's waits for its tensor-core work; its final drain always keeps
-                            the full limit. */
+                            at once (only used to test the timeout path).  The only such waits
+                            are the tcgen05 leaf Gram's for its tensor-core work, so any value
+                            but 0 selects that form; its final drain always keeps the full
+                            limit.  Results are identical either way. */
   int join_ctas_per_sm;  /* 0: the autotuner picks the NN-Descent kernel variant; 3 or 4 with
                             join_cblock 2, 4 or 8 forces that variant (resident CTAs per SM x
                             Hamming candidates in flight) for every iteration and for
@@ -100,7 +102,8 @@ typedef struct knng_params {
   int forest_fuse;       /* 1 (default): with native pivots, forest nodes of >= 512 members
                             are split three levels per pass over their code rows, the
                             descendants' pivots drawn from a seeded, evaluated sample of the
-                            node's members; 0: one level per pass.  A replay table
+                            node's members, and smaller nodes down to their leaves by one
+                            kernel; 0: one level per pass.  A replay table
                             (knng_forest) always splits one level per pass. */
 } knng_params;
 
@@ -118,7 +121,7 @@ typedef struct knng_stats {
   int64_t forest_levels;
   int64_t leaves;
   double device_s;        /* first to last device event of the call */
-  double join_ms[64];     /* device time of each NN-Descent launch */
+  double join_ms[64];     /* device time of each NN-Descent iteration */
   int64_t join_candidates[64]; /* sketches scored per iteration (distinct candidates without a
                                   cached score) */
   int64_t join_dots[64];  /* int8 rows reranked per iteration */

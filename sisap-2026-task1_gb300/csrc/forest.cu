@@ -19,7 +19,7 @@
 // A batch of jobs is one problem of N rows (tree-major [T][N] arrays, job b at
 // offset off[b] in every tree); every level serves all jobs' nodes at once.
 //
-// Per level: pick_pivots -> scan(tiles) -> side (8 lanes per row, dp4a,
+// Per level (replay, or fusing off): pick_pivots -> scan(tiles) -> side (8 lanes per row, dp4a,
 // HBM-bound: d bytes read per active member) -> scan(left counts) -> scatter
 // (stable partition into perm_tmp) -> copy back -> children (leaf flags,
 // next node list).
@@ -65,7 +65,7 @@ constexpr int kFuse = 3;                        // levels per fused pass
 constexpr int kFuseNodes = (1 << kFuse) - 1;    // split nodes of one fused subtree (depth 0 .. kFuse-1)
 constexpr int kFuseBins = 1 << kFuse;           // path codes
 constexpr int kCand = 64;                       // pivot candidates per fused node
-constexpr int32_t kFuseMin = 512;               // smaller nodes take the per-level path
+constexpr int32_t kFuseMin = 512;               // smaller nodes are left to subtree_kernel
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
@@ -739,7 +739,9 @@ __global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __re
 // part of the permutation in shared memory.  8 lanes per member and level: the
 // member's row is read (by then from L2, for the most part), the pivot rows
 // are staged in shared memory while at most kSubStage descendants are open
-// (with the default leaf size at most 7 are).  It replaces 10 to 16 rounds of
+// (with the default leaf size at most 7 are).  Bound by those reads: the
+// shared-memory pipe is 76 % busy at 300k x 1024 (1.78 ms); a warp per four
+// members with the pivots in registers made the forest 3 to 20 % slower.  It replaces 10 to 16 rounds of
 // 8 to 10 launches and two host waits each: with the wider fuse_pivots and one
 // wait per fused round the forest went from 0.97 to 0.24 ms at 2,000 x 384,
 // 4.71 to 2.66 ms at 100,000 x 1024 and 34.2 to 26.0 ms at 1M x 1024.
