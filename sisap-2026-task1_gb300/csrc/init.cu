@@ -171,7 +171,8 @@ __device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a > b
 // (init_merge): a leaf half gives 6 on average, and a merge costs about 300
 // instructions for 1 or 32.  Bound by instructions; with a merge per leaf half
 // and ranks by counting the initial graph took 4.17 ms at 300k x 1024 and
-// 14.9 at 1M, now 3.54 and 13.3 (waiting alone, ranks by counting: 4.07, 15.0).
+// 14.9 at 1M, with the sort 3.54 and 13.3 (waiting alone, ranks by counting:
+// 4.07, 15.0).
 __device__ __forceinline__ uint64_t merge_batch(uint64_t& kA, uint64_t& kB, uint64_t key, uint64_t thr, int K,
                                                 int lane, uint64_t* sl) {
   const unsigned full = 0xffffffffu;
@@ -223,86 +224,95 @@ __device__ __forceinline__ uint64_t merge_batch(uint64_t& kA, uint64_t& kB, uint
 // chunks from the list the previous chunk wrote (keys round-trip exactly, and
 // an empty entry, id -1 / INT32_MIN, is key 0), so the chunks give the list of
 // all trees at once.  Gram rows are stored from position gram_pos0 on.
-__global__ void __launch_bounds__(256) init_merge(int64_t n, int t0, int t1, int K, int first, int last,
-                                                  const int32_t* __restrict__ perm,
-                                                  const int32_t* __restrict__ pos,
-                                                  const int32_t* __restrict__ leaf_lo,
-                                                  const uint8_t* __restrict__ leaf_sz,
-                                                  const int32_t* __restrict__ gram, int64_t gram_pos0,
-                                                  int32_t* __restrict__ ids, int32_t* __restrict__ scores,
-                                                  int32_t* __restrict__ fix_rows, int64_t* __restrict__ fix_count,
-                                                  int64_t gram_rows, unsigned* err) {
+// A warp ends with its row: a grid that stays and strides over the rows took
+// 6 % longer.  Eight CTAs per SM (32 registers) and both halves' loads ahead of
+// the first merge gave 5 %: initial graph 3.23 ms at 300k, 11.5 at 1M.
+__global__ void __launch_bounds__(256, 8) init_merge(int64_t n, int t0, int t1, int K, int first, int last,
+                                                     const int32_t* __restrict__ perm,
+                                                     const int32_t* __restrict__ pos,
+                                                     const int32_t* __restrict__ leaf_lo,
+                                                     const uint8_t* __restrict__ leaf_sz,
+                                                     const int32_t* __restrict__ gram, int64_t gram_pos0,
+                                                     int32_t* __restrict__ ids, int32_t* __restrict__ scores,
+                                                     int32_t* __restrict__ fix_rows, int64_t* __restrict__ fix_count,
+                                                     int64_t gram_rows, unsigned* err) {
   (void)gram_rows;
   (void)err;
   __shared__ uint64_t s_list[8][kMaxK + 64];  // per warp: its list, then the waiting candidates
   uint64_t* const sl = s_list[threadIdx.x >> 5];
   uint64_t* const wait = sl + kMaxK;
   const int lane = threadIdx.x & 31;
-  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t i = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    uint64_t kA = 0, kB = 0, thr = 0;
-    if (!first) {
-      if (lane < K) {
-        const int32_t id = ids[i * K + lane];
-        kA = id >= 0 ? make_key(scores[i * K + lane], id) : 0;
-      }
-      if (32 + lane < K) {
-        const int32_t id = ids[i * K + 32 + lane];
-        kB = id >= 0 ? make_key(scores[i * K + 32 + lane], id) : 0;
-      }
-      thr = (K - 1) < 32 ? __shfl_sync(0xffffffffu, kA, K - 1) : __shfl_sync(0xffffffffu, kB, K - 33);
-    }
-    __syncwarp();
-    sl[lane] = kA;
-    sl[32 + lane] = kB;
-    __syncwarp();
-    int nw = 0;  // waiting candidates, fewer than 32 between halves
-    for (int t = t0; t < t1; ++t) {
-      const int64_t p = pos[int64_t(t) * n + i];
-      // (bounds-checked build) the position lies in tree t, its leaf in the
-      // same tree, and its Gram row in this chunk's rows
-      if (!KNNG_GUARD(err, p >= int64_t(t) * n && p < int64_t(t + 1) * n && p - gram_pos0 < gram_rows)) continue;
-      const int64_t s = leaf_lo[p];
-      const int m = leaf_sz[p];
-      if (!KNNG_GUARD(err, s >= int64_t(t) * n && s <= p && s + m <= int64_t(t + 1) * n && p < s + m)) continue;
-      const int self = int(p - s);
-      const int32_t* grow = gram + (p - gram_pos0) * int64_t(kMaxLeaf);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        if (32 * half >= m) break;  // warp-uniform
-        const int j = lane + 32 * half;
-        uint64_t key = 0;
-        if (j < m && j != self) key = make_key(grow[j], perm[s + j]);
-        const unsigned above = __ballot_sync(0xffffffffu, key > thr);
-        if (key > thr) wait[nw + __popc(above & ((1u << lane) - 1u))] = key;
-        nw += __popc(above);
-        if (nw >= 32) {
-          __syncwarp();
-          const uint64_t k0 = wait[lane], k1 = wait[32 + lane];  // k1: the first nw - 32 count
-          __syncwarp();
-          nw -= 32;
-          thr = merge_batch(kA, kB, k0, thr, K, lane, sl);
-          if (lane < nw) wait[lane] = k1;
-        }
-      }
-    }
-    __syncwarp();
-    thr = merge_batch(kA, kB, lane < nw ? wait[lane] : 0, thr, K, lane, sl);
-    const int real = __popc(__ballot_sync(0xffffffffu, kA != 0)) + __popc(__ballot_sync(0xffffffffu, kB != 0));
-    int32_t* gi = ids + i * K;
-    int32_t* gs = scores + i * K;
+  const int64_t i = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (i >= n) return;
+  uint64_t kA = 0, kB = 0, thr = 0;
+  if (!first) {
     if (lane < K) {
-      gi[lane] = kA ? key_id(kA) : -1;
-      gs[lane] = kA ? key_score(kA) : kScoreMinI;
+      const int32_t id = ids[i * K + lane];
+      kA = id >= 0 ? make_key(scores[i * K + lane], id) : 0;
     }
     if (32 + lane < K) {
-      gi[32 + lane] = kB ? key_id(kB) : -1;
-      gs[32 + lane] = kB ? key_score(kB) : kScoreMinI;
+      const int32_t id = ids[i * K + 32 + lane];
+      kB = id >= 0 ? make_key(scores[i * K + 32 + lane], id) : 0;
     }
-    if (last && real < K && lane == 0) {
-      const int64_t slot = atomicAdd(reinterpret_cast<unsigned long long*>(fix_count), 1ull);
-      fix_rows[slot] = int32_t(i);
+    thr = (K - 1) < 32 ? __shfl_sync(0xffffffffu, kA, K - 1) : __shfl_sync(0xffffffffu, kB, K - 33);
+  }
+  __syncwarp();
+  sl[lane] = kA;
+  sl[32 + lane] = kB;
+  __syncwarp();
+  int nw = 0;  // waiting candidates, fewer than 32 between halves
+  for (int t = t0; t < t1; ++t) {
+    const int64_t p = pos[int64_t(t) * n + i];
+    // (bounds-checked build) the position lies in tree t, its leaf in the
+    // same tree, and its Gram row in this chunk's rows
+    if (!KNNG_GUARD(err, p >= int64_t(t) * n && p < int64_t(t + 1) * n && p - gram_pos0 < gram_rows)) continue;
+    const int64_t s = leaf_lo[p];
+    const int m = leaf_sz[p];
+    if (!KNNG_GUARD(err, s >= int64_t(t) * n && s <= p && s + m <= int64_t(t + 1) * n && p < s + m)) continue;
+    const int self = int(p - s);
+    const int32_t* grow = gram + (p - gram_pos0) * int64_t(kMaxLeaf);
+    int32_t g2[2], q2[2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int j = lane + 32 * half;
+      g2[half] = j < m ? grow[j] : 0;
+      q2[half] = j < m ? perm[s + j] : 0;
     }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (32 * half >= m) break;  // warp-uniform
+      const int j = lane + 32 * half;
+      uint64_t key = 0;
+      if (j < m && j != self) key = make_key(g2[half], q2[half]);
+      const unsigned above = __ballot_sync(0xffffffffu, key > thr);
+      if (key > thr) wait[nw + __popc(above & ((1u << lane) - 1u))] = key;
+      nw += __popc(above);
+      if (nw >= 32) {
+        __syncwarp();
+        const uint64_t k0 = wait[lane], k1 = wait[32 + lane];  // k1: the first nw - 32 count
+        __syncwarp();
+        nw -= 32;
+        thr = merge_batch(kA, kB, k0, thr, K, lane, sl);
+        if (lane < nw) wait[lane] = k1;
+      }
+    }
+  }
+  __syncwarp();
+  thr = merge_batch(kA, kB, lane < nw ? wait[lane] : 0, thr, K, lane, sl);
+  const int real = __popc(__ballot_sync(0xffffffffu, kA != 0)) + __popc(__ballot_sync(0xffffffffu, kB != 0));
+  int32_t* gi = ids + i * K;
+  int32_t* gs = scores + i * K;
+  if (lane < K) {
+    gi[lane] = kA ? key_id(kA) : -1;
+    gs[lane] = kA ? key_score(kA) : kScoreMinI;
+  }
+  if (32 + lane < K) {
+    gi[32 + lane] = kB ? key_id(kB) : -1;
+    gs[32 + lane] = kB ? key_score(kB) : kScoreMinI;
+  }
+  if (last && real < K && lane == 0) {
+    const int64_t slot = atomicAdd(reinterpret_cast<unsigned long long*>(fix_count), 1ull);
+    fix_rows[slot] = int32_t(i);
   }
 }
 
@@ -678,7 +688,7 @@ int run_init(const int8_t* codes, int64_t n, int d, int T, int leaf, int K, uint
       }
     }
     cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
-    init_merge<<<unsigned(std::min<int64_t>((n + 7) / 8, int64_t(sms) * 16)), 256, 0, s>>>(
+    init_merge<<<unsigned((n + 7) / 8), 256, 0, s>>>(
         n, t0, t1, K, t0 == 0 ? 1 : 0, t1 == T ? 1 : 0, perm, ib.pos, ib.leaf_lo, ib.leaf_sz, ib.gram, pos0, ids,
         scores, ib.fix_rows, ib.dev_i64 + 1, int64_t(t1 - t0) * n, gerr);
     note_launch();
