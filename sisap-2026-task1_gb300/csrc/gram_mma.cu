@@ -30,10 +30,11 @@
 // DRAM reads, 0.38 of the DRAM peak, tensor pipe 0.33 busy.  What is left is
 // the latency of a segment's loads at 12 warps per SM (168 registers hold the
 // accumulators); prefetching the next leaf's rows into L2 and loading a
-// segment ahead changed it by less than 2 %, four CTAs per SM spilled.
+// segment ahead changed it by less than 2 %, four CTAs per SM spilled.  A warp
+// ends with its leaf: a grid that stayed and strode over the leaves, the next
+// leaf's ids loaded ahead, made the initial graph 2 % slower at 300k (3.17 ->
+// 3.23 ms) and 8 % at 1M (10.7 -> 11.6).
 #include "knng_internal.cuh"
-
-#include <algorithm>
 
 namespace knng {
 namespace {
@@ -134,50 +135,36 @@ __global__ void __launch_bounds__(kGmThreads, kGmCtas) leaf_gram_mma(const int8_
   (void)n_rows;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-  const int64_t stride = int64_t(gridDim.x) * kGmWarps;
-  int64_t l = int64_t(blockIdx.x) * kGmWarps + (threadIdx.x >> 5);
-  // extent of the next leaf and its member ids (2 per lane), loaded while the
-  // leaf before is computed
-  int64_t ns = 0;
-  int nm = 0;
-  int32_t nid0 = 0, nid1 = 0;
-  auto load_leaf = [&](int64_t q) {
-    nm = 0;
-    if (q >= nleaves) return;
-    ns = leaf_start[q];
-    nm = int((q + 1 < nleaves ? int64_t(leaf_start[q + 1]) : total) - ns);
-    nm = nm < kMaxLeaf ? nm : kMaxLeaf;  // (a leaf holds at most kMaxLeaf members)
-    if (lane < nm) nid0 = perm[ns + lane];
-    if (32 + lane < nm) nid1 = perm[ns + 32 + lane];
-  };
-  load_leaf(l);
-  for (; l < nleaves; l += stride) {
-    const int64_t s = ns;
-    const int m = nm;
-    // row 8i + g of this lane, the last member's in the rows past the end
-    // (their results are not stored)
-    int32_t id[kGroups];
+  const int64_t l = int64_t(blockIdx.x) * kGmWarps + (threadIdx.x >> 5);
+  if (l >= nleaves) return;
+  const int64_t s = leaf_start[l];
+  int m = int((l + 1 < nleaves ? int64_t(leaf_start[l + 1]) : total) - s);
+  m = m < kMaxLeaf ? m : kMaxLeaf;  // (a leaf holds at most kMaxLeaf members)
+  int32_t id0 = 0, id1 = 0;         // the leaf's member ids, 2 per lane
+  if (lane < m) id0 = perm[s + lane];
+  if (32 + lane < m) id1 = perm[s + 32 + lane];
+  // row 8i + g of this lane, the last member's in the rows past the end
+  // (their results are not stored)
+  int32_t id[kGroups];
 #pragma unroll
-    for (int i = 0; i < kGroups; ++i) {
-      const int r = max(min(8 * i + g, m - 1), 0);
-      const int32_t lo = __shfl_sync(full, nid0, r & 31), hi = __shfl_sync(full, nid1, r & 31);
-      id[i] = r < 32 ? lo : hi;
-      if (!KNNG_GUARD(err, id[i] >= 0 && id[i] < n_rows)) id[i] = 0;
-    }
-    load_leaf(l + stride);
-    const int8_t* base = codes + 16 * c;
-    int32_t* out = gram + (s - gram_pos0) * int64_t(kMaxLeaf);
-    switch ((m + 7) >> 3) {  // warp-uniform
-      case 1:
-      case 2: leaf_block<2>(base, id, d, m, g, c, out); break;
-      case 3:
-      case 4: leaf_block<4>(base, id, d, m, g, c, out); break;
-      case 5: leaf_block<5>(base, id, d, m, g, c, out); break;
-      case 6: leaf_block<6>(base, id, d, m, g, c, out); break;
-      case 7: leaf_block<7>(base, id, d, m, g, c, out); break;
-      case 8: leaf_block<8>(base, id, d, m, g, c, out); break;
-      default: break;
-    }
+  for (int i = 0; i < kGroups; ++i) {
+    const int r = max(min(8 * i + g, m - 1), 0);
+    const int32_t lo = __shfl_sync(full, id0, r & 31), hi = __shfl_sync(full, id1, r & 31);
+    id[i] = r < 32 ? lo : hi;
+    if (!KNNG_GUARD(err, id[i] >= 0 && id[i] < n_rows)) id[i] = 0;
+  }
+  const int8_t* base = codes + 16 * c;
+  int32_t* out = gram + (s - gram_pos0) * int64_t(kMaxLeaf);
+  switch ((m + 7) >> 3) {  // warp-uniform
+    case 1:
+    case 2: leaf_block<2>(base, id, d, m, g, c, out); break;
+    case 3:
+    case 4: leaf_block<4>(base, id, d, m, g, c, out); break;
+    case 5: leaf_block<5>(base, id, d, m, g, c, out); break;
+    case 6: leaf_block<6>(base, id, d, m, g, c, out); break;
+    case 7: leaf_block<7>(base, id, d, m, g, c, out); break;
+    case 8: leaf_block<8>(base, id, d, m, g, c, out); break;
+    default: break;
   }
 }
 
@@ -185,10 +172,10 @@ __global__ void __launch_bounds__(kGmThreads, kGmCtas) leaf_gram_mma(const int8_
 
 cudaError_t launch_leaf_gram_mma(const int8_t* codes, int d, const int32_t* perm, const int32_t* leaf_start,
                                  int64_t nleaves, int64_t total, int32_t* gram, int64_t gram_pos0, unsigned* err,
-                                 int num_sms, cudaStream_t s, int64_t n_rows) {
+                                 cudaStream_t s, int64_t n_rows) {
   if (d % 64 != 0) return cudaErrorInvalidValue;
   if (nleaves <= 0) return cudaSuccess;
-  const int64_t blocks = std::min<int64_t>((nleaves + kGmWarps - 1) / kGmWarps, int64_t(num_sms) * kGmCtas);
+  const int64_t blocks = (nleaves + kGmWarps - 1) / kGmWarps;  // below 2^31: num_trees * n is
   cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
   leaf_gram_mma<<<unsigned(blocks), kGmThreads, 0, s>>>(codes, d, perm, leaf_start, nleaves, total, gram, gram_pos0,
                                                         err, n_rows);

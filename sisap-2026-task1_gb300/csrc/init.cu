@@ -674,7 +674,7 @@ int run_init(const int8_t* codes, int64_t n, int d, int T, int leaf, int K, uint
       // the register form has no wait to bound: a caller that set a limit gets the
       // tcgen05 form, whose waits honour it
       if (gram_mode == 1 && wait_limit == 0) {
-        if ((e = launch_leaf_gram_mma(codes, d, perm, leaf_start + l0, l1 - l0, pos1, ib.gram, pos0, gerr, sms, s, n)))
+        if ((e = launch_leaf_gram_mma(codes, d, perm, leaf_start + l0, l1 - l0, pos1, ib.gram, pos0, gerr, s, n)))
           return fail(e, "tensor-core gram");
       } else if (gram_mode == 1) {
         if ((e = launch_leaf_gram_tc(codes, d, perm, leaf_start + l0, l1 - l0, pos1, ib.gram, pos0, gerr, sms, s,

@@ -223,7 +223,7 @@ cudaError_t launch_leaf_gram_tc(const int8_t* codes, int d, const int32_t* perm,
 // The same Gram rows by warp-level tensor-core instructions from registers (gram_mma.cu).
 cudaError_t launch_leaf_gram_mma(const int8_t* codes, int d, const int32_t* perm, const int32_t* leaf_start,
                                  int64_t nleaves, int64_t total, int32_t* gram, int64_t gram_pos0, unsigned* err,
-                                 int num_sms, cudaStream_t s, int64_t n_rows);
+                                 cudaStream_t s, int64_t n_rows);
 
 // Random initial graph (init_mode KNNG_INIT_RANDOM); every job needs n > K.
 cudaError_t launch_init_random(const int8_t* codes, int d, int64_t n_total, int K, uint32_t seed, const JobTable& jt,
