@@ -682,10 +682,11 @@ __global__ void __launch_bounds__(256) fuse_copyback(int32_t* __restrict__ perm,
 // counts; leaves are flagged, and every descendant that is neither a leaf nor
 // split in the pass becomes a node: of the next fused round when it has at
 // least kFuseMin members (with its tiles reserved), else parked for the
-// subtree kernel.  counts: nodes of the next round, their tiles, parked nodes.
+// subtree kernel, with its depth (the levels done when this round ends) in p1.
+// counts: nodes of the next round, their tiles, parked nodes.
 __global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __restrict__ bins_off,
                               const int32_t* __restrict__ piv, uint8_t* __restrict__ leaf_flag, int32_t* counts,
-                              NodeArr big, NodeArr small, int64_t cap, unsigned* err) {
+                              NodeArr big, NodeArr small, int32_t depth, int64_t cap, unsigned* err) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
   const int32_t start = nd.start[k], size = nd.size[k];
@@ -727,6 +728,7 @@ __global__ void fuse_children(NodeArr nd, int cnt, int leaf, const int32_t* __re
         } else {
           small.start[o] = int32_t(cstart);
           small.size[o] = csize;
+          small.p1[o] = depth;
         }
       }
     }
@@ -780,10 +782,12 @@ __global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__
     s_perm[0][t] = perm[int64_t(start) + t];
     s_node[t] = 0;
   }
-  int cnt = 1, cur = 0, level = level0;
+  // the valve counts from the node's own depth: a node of another tree or job
+  // that kept the fused rounds going (thousands of equal rows) does not close it
+  int cnt = 1, cur = 0, level = level0, depth = nd.p1[k0];
   __syncthreads();
   while (cnt > 0) {  // a level closes every node it splits; children are smaller: ends
-    if (level >= kMaxLevels) {  // depth valve: the rest become consecutive leaves
+    if (depth >= kMaxLevels) {  // depth valve: the rest become consecutive leaves
       for (int k = tid; k < cnt; k += 256)
         for (int p = s_start[cur][k], e = p + s_size[cur][k]; p < e; p += leaf) leaf_flag[int64_t(start) + p] = 1;
       break;
@@ -901,6 +905,7 @@ __global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__
     cnt = s_next;
     cur ^= 1;
     ++level;
+    ++depth;
   }
   for (int t = tid; t < size; t += 256) perm[int64_t(start) + t] = s_perm[cur][t];
   if (tid == 0) atomicMax(max_level, level);
@@ -1017,7 +1022,7 @@ int run_forest(const int8_t* codes, int64_t n, int d, int T, int leaf, uint32_t 
         return fail(e, "code scan");
       cudaGetLastError();  // clear a stale, non-sticky error: the launch reports only its own
       fuse_children<<<grid1(cnt, 64), 64, 0, s>>>(cur, int(cnt), leaf, fb.tile_bins_off, fb.piv, leaf_flag, counts, nxt,
-                                                  parked, fb.max_nodes, fb.err);
+                                                  parked, level + kFuse, fb.max_nodes, fb.err);
       note_launch();
       // the counts first: the next round is queued while the members are sorted
       if ((e = cudaMemcpyAsync(host_cnt, counts, sizeof(host_cnt), cudaMemcpyDeviceToHost, s)) ||
