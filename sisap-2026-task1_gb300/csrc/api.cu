@@ -129,9 +129,18 @@ struct knng_ctx {
 
 namespace {
 
-// Timed launches per configuration of an autotune sweep (the fastest counts).
-// The early iterations take most of the phase and their configurations lie
-// closest together, so theirs gets one more.
+// Timed launches per configuration of an autotune sweep (the fastest counts)
+// with the default K and R; any other K and R get one each.  The first build of
+// a bucket pays for them (first / repeated build): 20,011 x 768 15.9 / 2.4 ms,
+// 100,000 x 1024 47.8 / 13.1, 300,000 x 1024 70 / 47.5, 2,000,000 x 1024 564 /
+// 427; with the probing join of old and one launch each 16.9 / 5.7, 55.6 / 27.2,
+// 125 / 96, 1022 / 848.  The choice does not need the repeats (it flips between
+// forms whose builds take the same time to 0.3 % even so); the admission test of
+// the serving loop (tests/test_gpu_serve.py) does: it presumes that a first
+// build of 40,000 host rows still runs after 50 ms, and with two launches per
+// configuration that build takes 46 ms, with these 53.  For other K and R, three
+// and two launches made first builds slower than that join's (100,000 x 1024,
+// K = 20: 41.4 ms against 32.4).
 constexpr int kEarlyReps = 3, kLateReps = 2;
 constexpr int64_t kStageRows = 1 << 16;  // host-input rows per H2D chunk (256 MB at d = 1024)
 // byte offset in the context's 4096-byte scalar block of the bounds-checked
@@ -365,10 +374,13 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   // 4 far CTAs 45.5; 600,000 x 1024 clustered, first iteration: 33.7, 31.0, 28.7.
   const JoinForm with_far[] = {{4, 4, false}, {4, 8, false}, {4, 4, true}, {4, 8, true}, {4, 2, false}};
   const JoinForm general[] = {{4, 4, false}, {4, 8, false}, {3, 4, false}, {3, 8, false}, {4, 2, false}};
-  const auto& cand = join_has_far(p.k_build, p.k_build * p.rerank_mult) ? with_far : general;
+  const bool has_far = join_has_far(p.k_build, p.k_build * p.rerank_mult);
+  const auto& cand = has_far ? with_far : general;
   const int K = p.k_build;
-  // the sweeps process the first 1/16 of the rows (at least 64 per resident CTA),
-  // so tuning costs about one join launch on the first build of a bucket
+  // the sweeps process the first 1/16 of the rows (at least 64 per resident CTA):
+  // 11 launches, or 26 with the repeats of the default K and R (17 where only
+  // FAR forms are early candidates).  From 600,000 rows on they cost as much as
+  // one or two iterations of the join; up to 38,912 rows each is a whole one
   JoinCtl plain{};
   plain.row_limit = std::min<int64_t>(N, std::max<int64_t>(N / 16, int64_t(c->num_sms) * 4 * 64));
   JoinCtl cached = cache_ctl ? *cache_ctl : plain;
@@ -393,14 +405,14 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
       }
     return true;
   };
-  if (!sweep(&plain, far_early, kEarlyReps, &best.early)) return best;
+  if (!sweep(&plain, far_early, has_far ? kEarlyReps : 1, &best.early)) return best;
   best.late = best.early;
   if (cache_ctl) {
     if (cudaMemsetAsync(cache_ctl->cache_cnt, 0, size_t(N) * 4, c->stream) != cudaSuccess ||
         launch_join(c->codes.as<int8_t>(), c->join_sketch(), N, d, K, K * p.rerank_mult, ids[0], scs[0],
                     ids[1], scs[1], order, scratch_counters, c->num_sms, c->stream, nullptr, &cached,
                     best.early.ctas, best.early.cblock, c->sketch_words(d), best.early.far) != cudaSuccess ||
-        !sweep(&cached, false, kLateReps, &best.late))
+        !sweep(&cached, false, has_far ? kLateReps : 1, &best.late))
       return best;
   }
   c->tuned[key] = best;

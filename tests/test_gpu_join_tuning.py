@@ -1,0 +1,29 @@
+"""What the join's autotuner costs a context's first build.
+
+With use_graph = 0 two builds of the same rows launch the same kernels, so the
+first build of a (dimension, size) launches more by the tuner's sweeps alone.
+"""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _tuning_launches(knng, ctx, x):
+    counts = []
+    for _ in range(2):
+        st = knng.Stats()
+        ctx.build(x, stats=st)
+        counts.append(st.kernel_launches)
+    return counts[0] - counts[1]
+
+
+@pytest.mark.parametrize("k,mult", [(50, 4), (32, 8), (15, 4)])
+def test_other_sizes_are_tuned_by_one_launch_per_configuration(k, mult):
+    import knng
+    import synth
+
+    x = synth.mixture_torch(6001, 384, 60, 3)
+    with knng.Context(use_graph=0, k_build=k, rerank_mult=mult) as ctx:
+        # five configurations, a launch that fills the candidate cache, five with it
+        assert _tuning_launches(knng, ctx, x) == 11
+        assert _tuning_launches(knng, ctx, x) == 0
