@@ -23,6 +23,7 @@
 #include <thread>
 #include <cmath>
 #include <map>
+#include <tuple>
 
 namespace knng {
 namespace {
@@ -114,9 +115,9 @@ struct knng_ctx {
   // join phase captured as a CUDA graph, reused while the launch key matches
   cudaGraphExec_t join_graph = nullptr;
   std::vector<uintptr_t> join_graph_key;
-  // autotuned join configurations per (d, log2 rows): (ctas_per_sm, cblock) for
-  // the first two iterations and for the later, cache-served ones
-  std::map<std::pair<int, int>, JoinCfg> tuned;
+  // autotuned join forms per (d, log2 rows, codes beyond L2): join_far's line
+  // lies inside a bucket, and its two sides take different early forms
+  std::map<std::tuple<int, int, bool>, JoinCfg> tuned;
   std::vector<knng_ctx*> subs;  // contexts of the second and later dimension groups of a batch
   std::vector<DevBuf*> buffers() {
     return {&codes, &sketch, &graph, &perm, &leaf_flag, &scratch, &outbuf, &scalars, &jobs, &hsketch, &rowflags};
@@ -343,9 +344,9 @@ struct BJob {
 
 // Times the join configurations on the batch's initial graph (output to the
 // spare buffer, which iteration 0 overwrites) and keeps the fastest per
-// (d, log2 rows), on the first 1/16 of the rows in visit order.  The early
-// configuration is timed with no candidate cache;
-// with a cache (cache_ctl), one more launch fills every row's cache from the
+// (d, log2 rows, side of join_far's line), on the first 1/16 of the rows in
+// visit order.  The early configuration is timed with no candidate cache; with
+// a cache (cache_ctl), one more launch fills every row's cache from the
 // same graph and the configurations are timed again with all candidates
 // cached, which is what the later iterations look like.  The caller clears
 // the cache before the NN-Descent phase.
@@ -361,7 +362,7 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   // so the early form's far flag is not left to it.
   const bool far_early = join_far(N, d) && join_has_far(p.k_build, p.k_build * p.rerank_mult);
   best.early.far = far_early;
-  const auto key = std::make_pair(d, int(std::log2(double(N))));
+  const auto key = std::make_tuple(d, int(std::log2(double(N))), far_early);
   auto it = c->tuned.find(key);
   if (it != c->tuned.end()) return it->second;
   if (!p.autotune || p.join_mode != KNNG_JOIN_JACOBI) return best;
