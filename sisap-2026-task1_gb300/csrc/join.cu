@@ -170,7 +170,7 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
   const uint32_t kk = uint32_t(2 * s.pairs), r = uint32_t(R < s.KK ? R : s.KK);
   const uint32_t rounds = uint32_t(def ? (s.pairs + kThreads - 1) / kThreads : kMaxPairs);
   s.survivors = r;
-  s.kp = uint32_t(def ? K : kMaxK);
+  s.kp = uint32_t(K);
   // behind every occurrence index that a thread of the kernel forms
   s.dummy = rounds * kThreads * 2;
   uint32_t o = 0;
@@ -193,6 +193,11 @@ __host__ __device__ constexpr JoinLayout join_layout(int K, int R, int d, bool d
   return s;
 }
 static_assert(join_layout(kDefK, kDefR, kMaxDim, true, true).bytes <= 49072, "four FAR CTAs in 196 KB");
+// An SM's 228 KB hold four CTAs of 57,344 bytes each (and 1 KB of the system's),
+// 80 of them static.  With lists of kMaxK entries the general form missed the
+// fourth by 192 bytes at K = 50, R < 400, d = 1024: 100,000 rows, phase at
+// R = 350 / 200 / 50: 13.2 / 12.5 / 11.3 ms with three, 12.2 / 11.6 / 10.5 with four.
+static_assert(join_layout(kDefK, kDefR - kDefK, kMaxDim, false, false).bytes <= 57264, "four general CTAs at K = 50, R < 400");
 static_assert(join_layout(kDefK, kDefR, kMaxDim, true, true).ta_slots * 4 >= 14 * kDefR, "survivors in the first table");
 static_assert(kHBins * 4 >= kCacheCap * 2, "the histogram region stages the cached distances");
 
