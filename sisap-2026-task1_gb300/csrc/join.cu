@@ -1341,20 +1341,21 @@ using JoinKernel = void (*)(const int8_t*, const uint64_t*, int64_t, int, int, i
 
 // ctas_per_sm 3: up to 80 registers per thread, 3 resident CTAs; otherwise 64
 // registers, 4 resident CTAs.
-template <bool DEF, bool FAR>
+template <bool DEF>
 JoinKernel pick_variant(int ctas_per_sm, int cblock) {
   if (ctas_per_sm == 3)
-    return cblock == 2 ? join_kernel<2, 3, DEF, FAR> : cblock == 8 ? join_kernel<8, 3, DEF, FAR> : join_kernel<4, 3, DEF, FAR>;
-  return cblock == 2 ? join_kernel<2, 4, DEF, FAR> : cblock == 8 ? join_kernel<8, 4, DEF, FAR> : join_kernel<4, 4, DEF, FAR>;
+    return cblock == 2 ? join_kernel<2, 3, DEF, false> : cblock == 8 ? join_kernel<8, 3, DEF, false> : join_kernel<4, 3, DEF, false>;
+  return cblock == 2 ? join_kernel<2, 4, DEF, false> : cblock == 8 ? join_kernel<8, 4, DEF, false> : join_kernel<4, 4, DEF, false>;
 }
 // The kernel and shared-memory layout of a launch: the default K and R have
-// their own kernel, which reads the lists 8 bytes at a time (`aligned`).
+// their own kernel, which reads the lists 8 bytes at a time (`aligned`), and
+// its FAR form (four CTAs, 4 or 8 sketches in flight: what the tuner offers).
 JoinKernel variant(int K, int R, int d, bool aligned, int ctas_per_sm, int cblock, bool far, JoinLayout* L) {
   const bool def = K == kDefK && R == kDefR && aligned;
-  far = far && def;
+  far = far && def && ctas_per_sm == 4 && cblock != 2;
   *L = join_layout(K, R, def ? kMaxDim : d, def, far);
-  if (far) return pick_variant<true, true>(ctas_per_sm, cblock);
-  return def ? pick_variant<true, false>(ctas_per_sm, cblock) : pick_variant<false, false>(ctas_per_sm, cblock);
+  if (far) return cblock == 8 ? join_kernel<8, 4, true, true> : join_kernel<4, 4, true, true>;
+  return def ? pick_variant<true>(ctas_per_sm, cblock) : pick_variant<false>(ctas_per_sm, cblock);
 }
 
 bool join_has_far(int K, int R) { return K == kDefK && R == kDefR; }
@@ -1404,7 +1405,7 @@ const char* join_variant_error() { return g_variant_err; }
 cudaError_t join_prepare_all(int K, int R, int d) {
   for (int c : {3, 4})
     for (int b : {2, 4, 8})
-      for (bool far : {false, true}) {
+      for (bool far : {false, true}) {  // far only where variant() has such a form
         const cudaError_t e = join_prepare(K, R, d, c, b, far);
         if (e != cudaSuccess) return e;
       }
