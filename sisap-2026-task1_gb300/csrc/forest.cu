@@ -52,7 +52,7 @@
 //
 // Node lists are filled through atomic counters, so their order varies; a
 // node's pivots depend on its identity only, so the forest does not.
-#include "knng_internal.cuh"
+#include "f16_codes.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -488,9 +488,8 @@ __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t 
 
 // Member pass of the fused levels: one block per tile of <= 256 members of one
 // node.  Every member's dots with all of the node's (up to 14) pivot rows are
-// one tensor-core product, members x pivots, in f16 with fp32 accumulation:
-// codes are exact in f16 and every partial sum is an integer of magnitude <=
-// 2^24, so the dots are the exact int32 ones.  A warp takes 32 members (two
+// one tensor-core product, members x pivots, in f16 with fp32 accumulation,
+// which is exact (f16_codes.cuh).  A warp takes 32 members (two
 // mma.m16n8k16 row tiles) against 16 columns; a lane reads 16 consecutive
 // codes of its rows (the K order is free as long as the pivots follow it) and
 // widens them in registers; the pivots are widened once per block into shared
@@ -509,22 +508,6 @@ __global__ void __launch_bounds__(256) fuse_pivots(NodeArr nd, int cnt, int64_t 
 // the measured copy rate); all rounds at 1M 18.4 -> 13.5 ms.  Four CTAs per SM:
 // five spill (+15 %), three with a segment loaded ahead are 5 % slower.
 constexpr int kPivCols = 16;  // 14 pivots, two columns of zeros
-
-__device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {  // gram_tc.cu says how
-  const uint32_t u = w ^ 0x80808080u;
-  const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140);
-  const uint32_t b = __byte_perm(u, 0x64646464u, 0x4342);
-  asm("add.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(0xE480E480u));
-  asm("add.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(0xE480E480u));
-}
-
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 __global__ void __launch_bounds__(256, 4) fuse_side(const int8_t* __restrict__ codes, int d,
                                                     const int32_t* __restrict__ perm, NodeArr nd,

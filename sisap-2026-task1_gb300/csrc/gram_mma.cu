@@ -2,10 +2,9 @@
 // instructions straight from registers.
 //
 // Reference: the dots of src/main.cpp:261-269 (every pair of members of a
-// leaf).  Same arithmetic as leaf_gram_tc (gram_tc.cu): the int8 codes are
-// widened to f16, which holds them exactly, and multiplied into fp32
-// accumulators; every partial sum is an integer of magnitude <= 2^24, so the
-// result is the int32 dot bit for bit.
+// leaf).  Same arithmetic as leaf_gram_tc (gram_tc.cu): the int8 codes widened
+// to f16 and multiplied into fp32 accumulators, which gives the int32 dot bit
+// for bit (f16_codes.cuh).
 //
 // One warp per leaf.  For mma.m16n8k16 a thread's A registers of rows
 // 16R..16R+15 and its B registers of the same rows as columns hold the same
@@ -34,7 +33,7 @@
 // ends with its leaf: a grid that stayed and strode over the leaves, the next
 // leaf's ids loaded ahead, made the initial graph 2 % slower at 300k (3.17 ->
 // 3.23 ms) and 8 % at 1M (10.7 -> 11.6).
-#include "knng_internal.cuh"
+#include "f16_codes.cuh"
 
 namespace knng {
 namespace {
@@ -43,23 +42,6 @@ constexpr int kGmThreads = 128;
 constexpr int kGmWarps = kGmThreads / 32;
 constexpr int kGmCtas = 3;      // CTAs per SM: 168 registers per thread
 constexpr int kGroups = 8;      // 8-row groups of a leaf
-
-// Four int8 codes widened to two f16 pairs (gram_tc.cu says how).
-__device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-  const uint32_t u = w ^ 0x80808080u;
-  const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140);
-  const uint32_t b = __byte_perm(u, 0x64646464u, 0x4342);
-  asm("add.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(0xE480E480u));
-  asm("add.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(0xE480E480u));
-}
-
-__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // First tile of row tile R among G column groups: R-major, C = 2R..G-1.
 __host__ __device__ constexpr int tile_base(int R, int G) { return R * (G + 1 - R); }

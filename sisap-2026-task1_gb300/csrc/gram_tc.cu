@@ -36,7 +36,7 @@
 // whole block leaves together; the kernel then records kErrTimeout, waits for
 // its copies, lets thread 0 wait with the full limit for every MMA it
 // committed, and frees its tensor memory before returning.
-#include "knng_internal.cuh"
+#include "f16_codes.cuh"
 
 #include <algorithm>
 
@@ -85,18 +85,6 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 // Instruction descriptor, kind::f16: D f32, A and B f16 (type 0), both K-major, N, M.
 __host__ __device__ constexpr uint32_t instr_desc(int M, int N) {
   return (1u << 4) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
-}
-
-// Four int8 codes (one 32-bit word) widened to two f16 pairs, exactly and in
-// integer/packed-half steps: u = code + 128 (xor 0x80 per byte) becomes the f16
-// 1024 + u by placing 0x64 above each byte (0x6400 is 1024.0, whose unit in the
-// last place is 1), and one packed add of -1152 leaves code = u - 128.
-__device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-  const uint32_t u = w ^ 0x80808080u;
-  const uint32_t a = __byte_perm(u, 0x64646464u, 0x4140);  // codes 0, 1
-  const uint32_t b = __byte_perm(u, 0x64646464u, 0x4342);  // codes 2, 3
-  asm("add.f16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(0xE480E480u));
-  asm("add.f16x2 %0, %1, %2;" : "=r"(hi) : "r"(b), "r"(0xE480E480u));
 }
 
 // Byte offset of 16-byte piece pc (0..3) of row r in a ring slot: rows are

@@ -119,3 +119,25 @@ def test_batched_job_beside_equal_rows_equals_its_solo_build(env):
         np.testing.assert_array_equal(k, ks)
         np.testing.assert_array_equal(dd, ds)
         assert it == st.iterations
+
+
+def _extreme_codes(n, d, kind, seed):
+    rng = np.random.default_rng(seed)
+    if kind == "ends":  # dots up to d * 2^14 either way
+        codes = rng.choice(np.array([-128, 127, -1, 0, 1], np.int8), size=(n, d))
+        codes[: n // 8], codes[n // 8: n // 4] = -128, 127
+    else:  # dots of 0.99 * d * 2^14, a few units apart
+        codes = np.where(rng.random((n, d)) < 0.5, -127, -128).astype(np.int8)
+    return codes[rng.permutation(n)]
+
+
+@pytest.mark.parametrize("n,d,kind", [(3001, 1024, "ends"), (3001, 1024, "near"), (2000, 128, "ends"), (1300, 640, "near")])
+def test_forest_of_extreme_codes(env, n, d, kind):
+    """The member pass takes its dots in f16 with fp32 sums: exact up to 2^24, which 1024 codes of -128 reach."""
+    torch, knng = env
+    codes = _extreme_codes(n, d, kind, n + d)
+    ref_perm, ref_flags, _ = forest_with_valve(codes, 2, 64, 1337)
+    with knng.Context(num_trees=2) as ctx:
+        perm, flags = ctx.forest(torch.from_numpy(codes).cuda())
+    np.testing.assert_array_equal(perm.cpu().numpy(), ref_perm)
+    np.testing.assert_array_equal(flags.cpu().numpy(), ref_flags)
