@@ -607,7 +607,9 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
   };
   clear_tables();
   sts16(a_member + 2 * tid, 0);
-  uint32_t tag = kTagTop;           // block-uniform
+  // (bounds-checked build) few tags, so that a few rows wear them out
+  const uint32_t tag_top = kChecked ? uint32_t(KNNG_L(KK)) + 64u : kTagTop;
+  uint32_t tag = tag_top;           // block-uniform
   uint32_t par = 0;                 // parity of the computed rows
 
   // Bookkeeping of the last computed row, by thread 0 once a barrier has
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, MINB) join_kernel(
     }
     if (tag < uint32_t(KNNG_L(KK)) + 16u) {  // a row uses at most KK + 1 tags; block-uniform, once per ~300,000 rows
       clear_tables();
-      tag = kTagTop;
+      tag = tag_top;
       __syncthreads();
     }
     // ---- B  two-hop occurrences, pair p = tid + 256r holding j = 2p, 2p + 1;
