@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__
   __shared__ int32_t s_p1[kSubNodes], s_p2[kSubNodes];
   __shared__ int s_wcnt[16];
   __shared__ int s_next;
-  __shared__ int32_t s_local;
+  __shared__ int32_t s_local, s_depth;
   const unsigned full = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 7;
   const int k0 = blockIdx.x;
@@ -760,17 +760,20 @@ __global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__
     s_local = in_tree - jt.off[job_of(jt, in_tree)];
     s_start[0][0] = 0;
     s_size[0][0] = int16_t(size);
+    s_depth = nd.p1[k0];
   }
   for (int t = tid; t < size; t += 256) {
     s_perm[0][t] = perm[int64_t(start) + t];
     s_node[t] = 0;
   }
-  // the valve counts from the node's own depth: a node of another tree or job
-  // that kept the fused rounds going (thousands of equal rows) does not close it
-  int cnt = 1, cur = 0, level = level0, depth = nd.p1[k0];
+  // The valve counts from the node's own depth: a node of another tree or job
+  // that kept the fused rounds going (thousands of equal rows) does not close
+  // it.  The depth stays in shared memory: in a register beside the level it
+  // made some dimensions spill (500,009 x 768 8.00 -> 8.14 ms, here 8.02).
+  int cnt = 1, cur = 0, level = 0;
   __syncthreads();
   while (cnt > 0) {  // a level closes every node it splits; children are smaller: ends
-    if (depth >= kMaxLevels) {  // depth valve: the rest become consecutive leaves
+    if (level + s_depth >= kMaxLevels) {  // depth valve: the rest become consecutive leaves
       for (int k = tid; k < cnt; k += 256)
         for (int p = s_start[cur][k], e = p + s_size[cur][k]; p < e; p += leaf) leaf_flag[int64_t(start) + p] = 1;
       break;
@@ -888,10 +891,9 @@ __global__ void __launch_bounds__(256) subtree_kernel(const int8_t* __restrict__
     cnt = s_next;
     cur ^= 1;
     ++level;
-    ++depth;
   }
   for (int t = tid; t < size; t += 256) perm[int64_t(start) + t] = s_perm[cur][t];
-  if (tid == 0) atomicMax(max_level, level);
+  if (tid == 0) atomicMax(max_level, level0 + level);
 }
 
 template <int PL>
