@@ -371,8 +371,8 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
     return best;
   }
   // With a far form three CTAs are never the fastest: 300,000 x 1024 of
-  // 64-dimensional data, join of two iterations: 4 CTAs 62.7 ms, 3 CTAs 49.9,
-  // 4 far CTAs 45.5; 600,000 x 1024 clustered, first iteration: 33.7, 31.0, 28.7.
+  // 64-dimensional data, join of two iterations: 4 CTAs 63.2 ms, 3 CTAs 54.1,
+  // 4 far CTAs 45.6; 600,000 x 1024 clustered, first iteration: 33.8, 33.2, 28.6.
   const JoinForm with_far[] = {{4, 4, false}, {4, 8, false}, {4, 4, true}, {4, 8, true}, {4, 2, false}};
   const JoinForm general[] = {{4, 4, false}, {4, 8, false}, {3, 4, false}, {3, 8, false}, {4, 2, false}};
   const bool has_far = join_has_far(p.k_build, p.k_build * p.rerank_mult);
@@ -581,7 +581,7 @@ int run_batch(knng_ctx* c, BJob* jobs, int J, int d, knng_stats& S) {
   ctl.cache_cnt = nullptr;
   ctl.cache_cap = 0;
   ctl.row_limit = 0;  // every row
-  ctl.chg_in = nullptr;  // set per iteration by join_phase
+  ctl.chg_in = nullptr;  // set per iteration by join_iterations
   ctl.chg_out = nullptr;
   // the bounds-checked build's error word of the join and the export
   ctl.check_err = kChecked ? c->scalars.as<unsigned>(kCheckWord) : nullptr;

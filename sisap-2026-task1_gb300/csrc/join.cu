@@ -61,8 +61,8 @@
 // candidates are new, the gathers of sketches and code rows.  Forms that only
 // shorten latencies (next row's two-hop ids fetched early, two table losers per
 // step, wider threshold scans) changed nothing or cost 1 to 4 %.
-// 100,000 x 1024: the phase takes 9.8 ms (probing tables: 19.2), an iteration
-// of 300,000 x 1024 rows of 64-dimensional data 22.7 ms (46.6).
+// 100,000 x 1024: the phase takes 9.7 ms (probing tables: 19.8), two iterations
+// of 300,000 x 1024 rows of 64-dimensional data 45.6 ms (93.6).
 //
 // Stages per row (shared memory, K = 50, R = 400: 54 KB, FAR 48 KB); thread t
 // owns the occurrences j = 2p and 2p + 1 of the pairs p = t + 256r in every
@@ -135,7 +135,7 @@ constexpr int kDefK = 50, kDefR = 400;
 // leaves four CTAs 60 KB of L1 instead of 28.  Gathers in flight hold L1
 // lines, and with rows that come from beyond L2 there are many of them: at
 // 300,000 x 1024 (64-dimensional data) the first iteration reads the same
-// 113 GB of DRAM in 23.2 ms instead of 33.7.  It saves the space by keeping an
+// 113 GB of DRAM in 23.3 ms instead of 32.6.  It saves the space by keeping an
 // occurrence's info word and its pointer to the id's first occurrence in one
 // entry, and the survivors in the first table, at 2 % more instructions.
 

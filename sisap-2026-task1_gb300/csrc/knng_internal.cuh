@@ -237,8 +237,8 @@ cudaError_t launch_init_block(const int8_t* codes, int d, int64_t n_total, int K
 // ---- join.cu ----
 // Per-batch NN-Descent control block in device memory.
 struct JoinCtl {
-  unsigned long long* counters;   // [5]: updates, sketches scored, reranked rows, distinct candidates,
-                                  // rows skipped as unchanged
+  unsigned long long* counters;   // 8 per iteration: updates, sketches scored, reranked rows, distinct candidates,
+                                  // rows skipped as unchanged, three unused
   unsigned long long* job_upd;    // [count]: updates of this iteration per job
   int* job_done;                  // [count]: job stopped (its rows pass through)
   float* job_prev;                // [count]: previous iteration's update rate
