@@ -131,11 +131,12 @@ struct knng_ctx {
 namespace {
 
 // Timed launches per configuration of an autotune sweep (the fastest counts)
-// with the default K and R; any other K and R get one each.  The first build of
-// a bucket pays for them (first / repeated build): 20,011 x 768 15.9 / 2.4 ms,
-// 100,000 x 1024 47.8 / 13.1, 300,000 x 1024 70 / 47.5, 2,000,000 x 1024 564 /
-// 427; with the probing join of old and one launch each 16.9 / 5.7, 55.6 / 27.2,
-// 125 / 96, 1022 / 848.  The choice does not need the repeats (it flips between
+// with the default K and R, while a sweep covers the fewest rows that it may
+// (up to 622,592 rows); else one each.  The first build of a bucket pays for
+// them (first / repeated build): 20,011 x 768 15.9 / 2.4 ms, 100,000 x 1024
+// 47.8 / 13.1, 300,000 x 1024 70 / 47.5, 2,000,000 x 1024 503 / 427 (565 with
+// repeats), 6,350,000 x 1024 1878 / 1667 (2031); with the probing join of old
+// and one launch each 16.9 / 5.7, 55.6 / 27.2, 125 / 96, 1022 / 848.  The choice does not need the repeats (it flips between
 // forms whose builds take the same time to 0.3 % even so); the admission test of
 // the serving loop (tests/test_gpu_serve.py) does: it presumes that a first
 // build of 40,000 host rows still runs after 50 ms, and with two launches per
@@ -379,13 +380,14 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
   const auto& cand = has_far ? with_far : general;
   const int K = p.k_build;
   // the sweeps process the first 1/16 of the rows (at least 64 per resident CTA):
-  // 11 launches, or 26 with the repeats of the default K and R (17 where only
-  // FAR forms are early candidates).  From 600,000 rows on they cost as much as
-  // one or two iterations of the join; up to 38,912 rows each is a whole one
+  // 11 launches (8 where only FAR forms are early candidates), which from 622,593
+  // rows on cost about as much as an iteration of the join; below, with the
+  // repeats of the default K and R, 26 (17), each a whole join up to 38,912 rows
   JoinCtl plain{};
   plain.row_limit = std::min<int64_t>(N, std::max<int64_t>(N / 16, int64_t(c->num_sms) * 4 * 64));
   JoinCtl cached = cache_ctl ? *cache_ctl : plain;
   cached.row_limit = plain.row_limit;
+  const bool repeat = has_far && plain.row_limit > N / 16;
   auto sweep = [&](const JoinCtl* ctl, bool far_only, int reps, JoinForm* out) {
     float best_ms = 1e30f;
     for (int rep = 0; rep < reps; ++rep)
@@ -406,14 +408,14 @@ JoinCfg autotune_join(knng_ctx* c, int64_t N, int d, int32_t* const ids[2], int3
       }
     return true;
   };
-  if (!sweep(&plain, far_early, has_far ? kEarlyReps : 1, &best.early)) return best;
+  if (!sweep(&plain, far_early, repeat ? kEarlyReps : 1, &best.early)) return best;
   best.late = best.early;
   if (cache_ctl) {
     if (cudaMemsetAsync(cache_ctl->cache_cnt, 0, size_t(N) * 4, c->stream) != cudaSuccess ||
         launch_join(c->codes.as<int8_t>(), c->join_sketch(), N, d, K, K * p.rerank_mult, ids[0], scs[0],
                     ids[1], scs[1], order, scratch_counters, c->num_sms, c->stream, nullptr, &cached,
                     best.early.ctas, best.early.cblock, c->sketch_words(d), best.early.far) != cudaSuccess ||
-        !sweep(&cached, false, has_far ? kLateReps : 1, &best.late))
+        !sweep(&cached, false, repeat ? kLateReps : 1, &best.late))
       return best;
   }
   c->tuned[key] = best;

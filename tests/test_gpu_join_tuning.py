@@ -29,6 +29,16 @@ def test_other_sizes_are_tuned_by_one_launch_per_configuration(k, mult):
         assert _tuning_launches(knng, ctx, x) == 0
 
 
+def test_long_sweeps_are_not_repeated():
+    """Beyond 622,592 rows a sweep's launch covers 1/16 of them and takes milliseconds."""
+    import knng
+    import synth
+
+    x = synth.mixture_torch(640001, 128, 2000, 3)
+    with knng.Context(use_graph=0) as ctx:
+        assert _tuning_launches(knng, ctx, x) <= 11
+
+
 def test_tuning_of_a_size_does_not_depend_on_the_sizes_before():
     """82,000 and 123,000 rows of 1024 codes share a power of two, and join_far's line (120 MiB of
     codes) lies between them: each is tuned for itself, whichever is built first."""
